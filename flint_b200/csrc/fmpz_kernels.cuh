@@ -27,6 +27,8 @@ k_fmpz_crt(const uint32_t* __restrict__ res, int logM, uint64_t Ly, uint32_t S, 
            uint64_t zh, uint32_t zw, uint64_t* __restrict__ z, CrtConst K)
 {
     const uint64_t j = zl + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
     if (j >= zh) return;
     uint64_t* __restrict__ out = z + (j - zl) * zw;
     const uint64_t n0 = j * S;
@@ -74,6 +76,7 @@ k_fmpz_crt_tiled(const uint32_t* __restrict__ res, int logM, uint64_t Ly, uint32
 {
     __shared__ uint64_t sc0[FZ_CRT_POS], sc1[FZ_CRT_POS], sc2[FZ_CRT_POS];
     const uint64_t j0 = zl + (uint64_t)blockIdx.x * J;
+    pdl_wait();
     if (j0 >= zh) return;
     const uint32_t nj = (uint32_t)(zh - j0 < J ? zh - j0 : J);
     const uint64_t p0 = j0 * S;
@@ -93,6 +96,7 @@ k_fmpz_crt_tiled(const uint32_t* __restrict__ res, int logM, uint64_t Ly, uint32
         sc2[t] = c2;
     }
     __syncthreads();
+    pdl_trigger();
     for (uint32_t q = threadIdx.x; q < nj; q += blockDim.x) {
         uint64_t* __restrict__ out = z + (j0 + q - zl) * zw;
         const uint32_t base = q * S;

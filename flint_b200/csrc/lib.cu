@@ -585,6 +585,35 @@ static LaunchShape make_shape(int logM, int logC = -1)
     return L;
 }
 
+// Launch as a programmatic dependent of the kernel before it on the stream
+// (dep), or plainly.
+template <typename... P, typename... A>
+static void launch_dep(void (*f)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool dep, A... args)
+{
+    cudaLaunchConfig_t cfg{};
+    cudaLaunchAttribute at[1];
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = dep ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, f, P(args)...);
+}
+
+// Row kernels run as dependents of the forward column pass up to 2^20 points.
+// Beyond, they start while column CTAs still wait for their turn on an SM and
+// cost more than the gap they hide (products of n x n limbs, dependent against
+// plain row launch: 2^16 30.1 / 32.8 us, 2^18 78.3 / 80.3, 4 10^5 124.4 / 126.5;
+// 7 10^5, a 3 2^19-point transform, 202.6 / 198.5).  k_rows<14, 5> has no wait
+// compiled in (rows_dep) and never runs as one.
+static bool rows_dependent(size_t points, int logC, int loge = 5)
+{
+    return points <= (size_t)1 << 20 && (logC < LOG_MAXC || loge == 4);
+}
+
 // the three transform launches shared by every product type; with a batch
 // descriptor array (ninst products of this shape) a, b, ra, rb are ignored;
 // with fz the operands are integer polynomials (an, bn coefficients); with co
@@ -993,6 +1022,8 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
     // b's twist factors, so the row pass multiplies the spectra once instead
     // of twice; squarings keep the scale in the row pass.
     const bool fold = !(sq && !desc) && S.logR >= 5;
+    // a batch's launches are the nodes of its graph, without launch gaps
+    const bool dep = !desc;
     const int R = 1 << S.logR;
     if (b_ready && !desc && !sq) {
         // b is still arriving: a's column pass first, b's after its copy
@@ -1025,20 +1056,21 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
         }
     } else {
         if (b_ready) cudaStreamWaitEvent(st, b_ready, 0);
-        fwd<<<dim3(np, cf.grid, zdim), cf.threads, cf.smem, st>>>(X->T, a, an, b, bn, ra, rb, S.logC, cf.G, desc,
-                                                                  np, shape, d_scale, fold ? 2 : 0);
+        launch_dep(fwd, dim3(np, cf.grid, zdim), cf.threads, cf.smem, st, dep && (cf.narrow || S.logR < 5), X->T, a, an, b, bn, ra, rb, S.logC, cf.G,
+                   desc, np, shape, d_scale, fold ? 2 : 0);
     }
     timing_mark(tr, 1, st);
     const LaunchShape Lr = row_launch_shape(X, L, np, ni);
     const int items = Lr.row_grid * np * ni;
     const int loge = rows_loge(X, Lr, np, ni);
-    (loge == 4 ? ROWS16 : ROWS)[S.logC]<<<std::min(items, X->nsm * rows_per_sm(Lr, loge)),
-                                         (Lr.nv << S.logC) >> loge, Lr.row_smem, st>>>(
-        X->T, ra, rb, S.logR, Lr.nv, np, fold ? nullptr : d_scale, (sq && !desc) ? 1 : 0, desc, ni, R);
+    launch_dep((loge == 4 ? ROWS16 : ROWS)[S.logC], std::min(items, X->nsm * rows_per_sm(Lr, loge)),
+               (Lr.nv << S.logC) >> loge, Lr.row_smem, st,
+               dep && rows_dependent((size_t)1 << (S.logR + S.logC), S.logC, loge), X->T, ra, rb, S.logR, Lr.nv, np,
+               fold ? nullptr : d_scale, (sq && !desc) ? 1 : 0, desc, ni, R);
     timing_mark(tr, 2, st);
     if (S.logR > 0)
-        inv<<<dim3(ci.grid, np, ni), ci.threads, ci.smem, st>>>(X->T, ra, S.logC, ci.G, desc,
-                                                                co ? *co : ChunkOut{nullptr, 0, 0, 0, 0});
+        launch_dep(inv, dim3(ci.grid, np, ni), ci.threads, ci.smem, st, dep && S.logR < 9, X->T, ra, S.logC, ci.G, desc,
+                   co ? *co : ChunkOut{nullptr, 0, 0, 0, 0});
     timing_mark(tr, 3, st);
     return ra;
 }
@@ -1059,15 +1091,16 @@ static void launch_transforms3(const Ctx *X, int k, int logMs, const uint64_t *a
     const size_t smem = (size_t)(padw(3 * (1 << r) * G) + 32) * sizeof(uint32_t);
     const uint32_t *sc = scale3_ptr(X, k);
     if (b_ready) cudaStreamWaitEvent(st, b_ready, 0);
-    (fz ? FWD_COLS3_FZ : FWD_COLS3)[r - LOG3_RMIN]<<<dim3(np, C / G, sq ? 1 : 2), 512, smem, st>>>(
-        X->T, a, an, b, bn, ra, rb, logMs, k, sc, sq ? 0 : 2, fz ? *fz : FzShape{1, 1, 1});
+    launch_dep((fz ? FWD_COLS3_FZ : FWD_COLS3)[r - LOG3_RMIN], dim3(np, C / G, sq ? 1 : 2), 512, smem, st, !b_ready,
+               X->T, a, an, b, bn, ra, rb, logMs, k, sc, sq ? 0 : 2, fz ? *fz : FzShape{1, 1, 1});
     timing_mark(tr, 1, st);
     const LaunchShape L = make_shape(logMs, LOGC3);   // row launch shape (one 2^13-point row per item)
     const int items = rows * np;
-    ROWS[LOGC3]<<<std::min(items, X->nsm * rows_per_sm(L)), L.row_threads, L.row_smem, st>>>(
-        X->T, ra, rb, logMs - LOGC3, 1, np, sq ? sc : nullptr, sq ? 1 : 0, nullptr, 1, rows);
+    launch_dep(ROWS[LOGC3], std::min(items, X->nsm * rows_per_sm(L)), L.row_threads, L.row_smem, st,
+               rows_dependent((size_t)3 << k, LOGC3), X->T, ra, rb, logMs - LOGC3, 1, np, sq ? sc : nullptr, sq ? 1 : 0,
+               nullptr, 1, rows);
     timing_mark(tr, 2, st);
-    INV_COLS3[r - LOG3_RMIN]<<<dim3(C / G, np), 512, smem, st>>>(X->T, ra, logMs, k);
+    launch_dep(INV_COLS3[r - LOG3_RMIN], dim3(C / G, np), 512, smem, st, true, X->T, ra, logMs, k);
     timing_mark(tr, 3, st);
 }
 
@@ -1334,14 +1367,9 @@ static int mpn_mul_enqueue(Ctx *X, uint64_t *z, const uint64_t *a, uint64_t an,
     for (int c = 0; c < nch; c++) {
         const size_t t0 = tiles * c / nch, t1 = tiles * (c + 1) / nch;
         if (t1 == t0) continue;
-        if (np == 5)
-            k_crt_carry<5, THREADS><<<t1 - t0, THREADS, 0, st>>>(ra, logM, an + bn - 1, zn, z, K, X->d_status,
-                                                                X->d_ticket, X->ticket_base, X->epoch, X->d_err,
-                                                                nullptr, nullptr, base);
-        else
-            k_crt_carry<6, THREADS><<<t1 - t0, THREADS, 0, st>>>(ra, logM, an + bn - 1, zn, z, K, X->d_status,
-                                                                X->d_ticket, X->ticket_base, X->epoch, X->d_err,
-                                                                nullptr, nullptr, base);
+        launch_dep(np == 5 ? k_crt_carry<5, THREADS> : k_crt_carry<6, THREADS>, t1 - t0, THREADS, 0, st, nch == 1,
+                   ra, logM, an + bn - 1, zn, z, K, X->d_status, X->d_ticket, X->ticket_base, X->epoch, X->d_err,
+                   nullptr, nullptr, base);
         if (chunks && chunks->hook)
             chunks->hook(chunks->arg, base + t0 * TILE, std::min<uint64_t>(zn, base + t1 * TILE));
     }
@@ -2655,9 +2683,8 @@ int gpu_mpn_mul_device_noalloc(uint64_t *z_dev, const uint64_t *a_dev, gpu_ulong
         return GPU_FFT_SMALL_ECUDA;
     launch_transforms(&D.ctx, shape, NA_NP, a_dev, an, b_dev, bn, ra, rb, sq,
                       D.scale + (size_t)logM * MAX_NP, st, nullptr);
-    k_crt_carry<NA_NP, THREADS><<<tiles, THREADS, 0, st>>>(ra, logM, L, zn, z_dev, D.ctx.crt[NA_NP],
-                                                          D.status, D.ticket, 0ull, 1u, D.err,
-                                                          nullptr, nullptr, 0ull);
+    launch_dep(k_crt_carry<NA_NP, THREADS>, tiles, THREADS, 0, st, true, ra, logM, L, zn, z_dev, D.ctx.crt[NA_NP],
+               D.status, D.ticket, 0ull, 1u, D.err, nullptr, nullptr, 0ull);
     return cudaGetLastError() == cudaSuccess ? GPU_FFT_SMALL_OK : GPU_FFT_SMALL_ECUDA;
 }
 

@@ -136,6 +136,7 @@ k_fwd_cols3(DevTables T, const uint64_t* __restrict__ a, uint64_t an, const uint
     uint32_t* __restrict__ out = (opb ? rb : ra) + ((size_t)j << logMs);
     const PrimeInfo P = T.pi[j];
     const uint32_t p = P.p;
+    pdl_wait();
 
     // limbs of rows 0 .. 3R' - 1 (element n = u C + i; zero beyond the operand).
     // blockDim == 512: thread t loads rows u_t + k 512/G of its column, so its
@@ -226,6 +227,7 @@ k_fwd_cols3(DevTables T, const uint64_t* __restrict__ a, uint64_t an, const uint
         gs_contig<5, COL_FMA_ADDS>(xr, c_w32[j], p);
         const uint32_t col = (uint32_t)(i0 + v);
         twist32_3<LOGR>(xr, col, s, t, k, th3, tl3, P, fsc);
+        if (f + (int)blockDim.x >= 3 * G * NS) pdl_trigger();
         uint32_t* o = out + ((size_t)(t * RP + 32 * s) << LOGC3) + col;
 #pragma unroll
         for (int m = 0; m < 32; m++) o[m * C] = xr[m];
@@ -250,6 +252,8 @@ k_inv_cols3(DevTables T, uint32_t* __restrict__ ra, int logMs, int k)
     const uint2* __restrict__ th3 = T.th3i + (size_t)j * TH3_SZ;
     const uint2* __restrict__ tl3 = T.tl3i + (size_t)j * TL_SZ;
     constexpr int NS = RP / 32;
+    pdl_wait();
+    pdl_trigger();
     for (int f = threadIdx.x; f < 3 * G * NS; f += blockDim.x) {
         const int t = f / (G * NS), rem = f - t * (G * NS);
         const int v = rem & (G - 1), s = rem / G;

@@ -55,6 +55,21 @@ struct DevTables {
     const uint2* w3c;      // [NP3][2] (w - w^2, w^-1 - w^-2), w = w3^(2^25) of order 3
 };
 
+// Programmatic dependent launch.  A kernel launched as a programmatic
+// dependent (launch_dep in lib.cu) may start while its predecessor on the
+// stream still runs; pdl_wait() holds it until that predecessor has completed
+// and its writes are visible, pdl_trigger() lets the successor start.  Without
+// such a launch both do nothing.
+// A short product is a chain of three or four kernels of 3-12 us each, so
+// the launch gaps between them are a fifth of its time.  The forward column and
+// the CRT kernels trigger just before their stores, not at their start: the
+// row kernel's few CTAs, placed while all the column CTAs are still resident,
+// share SMs that would be free a moment later (2^15 x 2^15 limbs: 30.1 us
+// plain, 26.0 us with early triggers, 23.5 us with late ones; 2^11 x 2^11: 20.5,
+// 25.0, 13.6 us).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;"); }
+
 // w_M^e * x for e in units of the largest transform (e < 2^25)
 __device__ __forceinline__ uint32_t twist_mul(uint32_t x, uint32_t e, const uint2* __restrict__ th,
                                               const uint2* __restrict__ tl, uint32_t p)
@@ -194,6 +209,13 @@ __device__ __forceinline__ uint32_t load_residue(const uint64_t* __restrict__ x,
 // smem = padw(R * G) words.
 // LC != 0: the row length 2^LC is a compile-time constant (logC == LC), so
 // the strided stores take immediate offsets instead of address arithmetic.
+// Instances that may run as programmatic dependents: short columns and narrow
+// tiles, which only launches of a few CTAs per SM take.  The wide ones serve
+// large products, where a launch gap is nothing and the wait's memory barrier
+// costs the schedule of the loads (2^25-point forward pass 1.13 -> 1.5 ms with
+// it compiled in).
+template <int LOGR, int G>
+__device__ __host__ constexpr bool fwd_cols_dep() { return LOGR < 5 || G < cols_per_tile(LOGR); }
 template <int LOGR, int G, bool FZ, int LC>
 __device__ __forceinline__ void
 fwd_cols_body(DevTables T, const uint64_t* __restrict__ a, uint64_t an,
@@ -337,6 +359,7 @@ fwd_cols_body(DevTables T, const uint64_t* __restrict__ a, uint64_t an,
             gs_contig<5, COL_FMA_ADDS>(xr, c_w32[j], p);
             const uint32_t col = (uint32_t)(i0 + v);
             twist32<LOGR>(xr, col, s, logM, th, tl, P, fsc);
+            if constexpr (fwd_cols_dep<LOGR, G>()) pdl_trigger();
             // rows 32 s .. 32 s + 31 of column col: a pointer bump per row keeps
             // the address arithmetic on the ALU pipe (the FMA pipe is this
             // kernel's busiest unit)
@@ -385,6 +408,7 @@ k_fwd_cols(DevTables T, const uint64_t* __restrict__ a, uint64_t an,
            const InstDesc* __restrict__ desc, int np, FzShape fz, const uint32_t* __restrict__ fscale,
            int fmask)
 {
+    if constexpr (fwd_cols_dep<LOGR, G>()) pdl_wait();
     if (LC != 0 && logC == LC)
         fwd_cols_body<LOGR, G, FZ, LC>(T, a, an, b, bn, ra, rb, logC, gcols, desc, np, fz, fscale, fmask);
     else
@@ -471,6 +495,11 @@ __device__ __forceinline__ void rows_prefetch(uint32_t* dst, const uint32_t* __r
     cp_async_commit();
 }
 
+// 2^14-point rows at 32 points per thread run large products only, which gain
+// nothing from an early launch (1.474 ms; 1.483 ms with the wait compiled in).
+template <int LOGC, int LOGE>
+__device__ __host__ constexpr bool rows_dep() { return LOGC < LOG_MAXC || LOGE == 4; }
+
 template <int LOGC, int LOGE = 5>
 __global__ void __launch_bounds__(LOGE == 4 ? 1024 : 512, 1)
 k_rows(DevTables T, uint32_t* __restrict__ ra, const uint32_t* __restrict__ rb,
@@ -505,6 +534,10 @@ k_rows(DevTables T, uint32_t* __restrict__ ra, const uint32_t* __restrict__ rb,
     };
 
     int g = blockIdx.x;
+    if constexpr (rows_dep<LOGC, LOGE>()) {
+        pdl_wait();
+        pdl_trigger();
+    }
     if (g >= total) return;
     {
         int j, u0;
@@ -719,6 +752,11 @@ __global__ void __launch_bounds__(512)
 k_inv_cols(DevTables T, uint32_t* __restrict__ ra, int logC, int gcols,
            const InstDesc* __restrict__ desc, ChunkOut co)
 {
+    // as the forward pass: the constant-stride instances serve large products
+    if constexpr (LC == 0) {
+        pdl_wait();
+        pdl_trigger();
+    }
     inv_cols_body<LOGR, G, LC>(T, ra, logC, gcols, desc, co);
 }
 
@@ -946,6 +984,7 @@ k_crt_carry(const uint32_t* __restrict__ res, int logM, uint64_t L, uint64_t zn,
     __shared__ uint32_t wg[NW], wp[NW];
     __shared__ uint32_t sh_carry_in;
 
+    pdl_wait();
     if (threadIdx.x == 0) sh_tile = (uint32_t)(atomicAdd(ticket, 1ull) - ticket_base);
     __syncthreads();
     // `gtile` numbers tiles across the launch (status words, look-back order);
@@ -1131,6 +1170,7 @@ k_crt_carry(const uint32_t* __restrict__ res, int logM, uint64_t L, uint64_t zn,
         sh_carry_in = cin;
     }
     __syncthreads();
+    pdl_trigger();
     uint32_t c = Ge | (Pe & sh_carry_in);
     uint64_t v[PER];
 #pragma unroll

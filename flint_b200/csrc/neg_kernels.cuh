@@ -54,6 +54,8 @@ __global__ void k_neg_split(DevTables T, const uint64_t* __restrict__ x, uint32_
     const uint32_t m = 1u << sh.logm;
     const uint64_t total = (uint64_t)count << sh.logm;
     const uint32_t b = sh.b;
+    pdl_wait();
+    pdl_trigger();
     for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t prod = (uint32_t)(e >> sh.logm), i = (uint32_t)e & (m - 1);
@@ -90,6 +92,8 @@ __global__ void k_neg_pointwise(DevTables T, uint32_t* __restrict__ X, const uin
 {
     const uint64_t per = (uint64_t)count << logm;
     const uint64_t total = per * np;
+    pdl_wait();
+    pdl_trigger();
     for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (uint64_t)gridDim.x * blockDim.x) {
         const int k = (int)(e / per);
@@ -181,6 +185,8 @@ k_neg_finish(DevTables T, const uint32_t* __restrict__ buf, const uint32_t* __re
     const size_t pstride = (size_t)1 << (sh.logR + sh.logm);
     const uint32_t* __restrict__ rp = buf + ((size_t)prod << sh.logm);
     if (t == 0) s_cin = 0;
+    pdl_wait();
+    pdl_trigger();
     __syncthreads();
 
     for (uint32_t J = 0; J < whi; J += Q.tl) {

@@ -58,6 +58,8 @@ k_crt_nmod(const uint32_t* __restrict__ res, int logM, uint64_t zl, uint64_t zh,
            uint64_t* __restrict__ z, CrtConst K, NmodConst N)
 {
     const uint64_t k = zl + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_wait();
+    pdl_trigger();
     if (k >= zh) return;
     uint64_t c0, c1, c2;
     const uint64_t pos = k & (((uint64_t)1 << logM) - 1);

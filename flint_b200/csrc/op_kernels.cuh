@@ -35,6 +35,8 @@ k_rows_fwd(DevTables T, uint32_t* __restrict__ buf, int logR, int nv, int np, in
     const int t = threadIdx.x;
     const int pb = (t / NSUB) * PC + 33 * (t & (NSUB - 1));
     uint32_t* __restrict__ base = buf + ((size_t)j << logM);
+    pdl_wait();
+    pdl_trigger();
     rows_prefetch<LOGC>(sm, base, u0, nv, R);
     cp_async_wait<0>();
     __syncthreads();
@@ -73,6 +75,8 @@ k_rows_inv(DevTables T, uint32_t* __restrict__ buf, int logR, int nv, int np, in
     const int t = threadIdx.x;
     const int pb = (t / NSUB) * PC + 33 * (t & (NSUB - 1));
     uint32_t* __restrict__ base = buf + ((size_t)j << logM);
+    pdl_wait();
+    pdl_trigger();
     rows_prefetch<LOGC>(sm, base, u0, nv, R);
     cp_async_wait<0>();
     __syncthreads();
@@ -103,6 +107,8 @@ __global__ void k_op_pointwise(DevTables T, int op, uint32_t* __restrict__ Z, co
 {
     const size_t M = (size_t)1 << logM;
     const size_t total = M * np;
+    pdl_wait();
+    pdl_trigger();
     for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (size_t)gridDim.x * blockDim.x) {
         const int j = (int)(e >> logM);
