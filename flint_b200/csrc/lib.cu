@@ -12,6 +12,7 @@
 #include "op_kernels.cuh"
 #include "neg_kernels.cuh"
 #include "mpn3_kernels.cuh"
+#include "rows_tc_kernels.cuh"
 
 #include <cuda_runtime.h>
 #include <math.h>
@@ -357,6 +358,14 @@ static int ctx_build_tables(Ctx *X)
         w3c[(size_t)j * 2] = shoup_pair(c, p);
         w3c[(size_t)j * 2 + 1] = shoup_pair(ci, p);
     }
+    // matrices and quotient constants of the tensor-core transforms
+    std::vector<uint8_t> tcw((size_t)TC_W_BYTES * MAX_NP);
+    std::vector<TcPrime> tcp(MAX_NP);
+    for (int j = 0; j < MAX_NP; j++) {
+        const uint32_t p = PRIMES[j];
+        tc_fill_w(&tcw[(size_t)j * TC_W_BYTES], h_powmod(primitive_root(p), (p - 1) >> 5, p), p);
+        tcp[j] = tc_prime(p);
+    }
     // CRT constants for every prime count
     for (int np = 1; np <= MAX_NP; np++) {
         CrtConst &K = X->crt[np];
@@ -383,6 +392,7 @@ static int ctx_build_tables(Ctx *X)
     const size_t o_th3i = place(sizeof(uint2) * n_th3), o_tl3i = place(sizeof(uint2) * n_tl3);
     const size_t o_tw3f = place(sizeof(uint2) * n_tw3), o_tw3i = place(sizeof(uint2) * n_tw3);
     const size_t o_w3c = place(sizeof(uint2) * NP3 * 2);
+    const size_t o_tcw = place((size_t)TC_W_BYTES * MAX_NP), o_tcp = place(sizeof(TcPrime) * MAX_NP);
     CU(cudaMalloc(&X->d_tables, off));
     char *base = (char *)X->d_tables;
     CU(cudaMemcpy(base + o_pi, pi.data(), sizeof(PrimeInfo) * MAX_NP, cudaMemcpyHostToDevice));
@@ -399,6 +409,10 @@ static int ctx_build_tables(Ctx *X)
     CU(cudaMemcpy(base + o_tw3f, tw3f.data(), sizeof(uint2) * n_tw3, cudaMemcpyHostToDevice));
     CU(cudaMemcpy(base + o_tw3i, tw3i.data(), sizeof(uint2) * n_tw3, cudaMemcpyHostToDevice));
     CU(cudaMemcpy(base + o_w3c, w3c.data(), sizeof(uint2) * NP3 * 2, cudaMemcpyHostToDevice));
+    CU(cudaMemcpy(base + o_tcw, tcw.data(), tcw.size(), cudaMemcpyHostToDevice));
+    CU(cudaMemcpy(base + o_tcp, tcp.data(), sizeof(TcPrime) * MAX_NP, cudaMemcpyHostToDevice));
+    X->T.tcw = (const uint4 *)(base + o_tcw);
+    X->T.tcp = (const TcPrime *)(base + o_tcp);
     X->T.pi = (const PrimeInfo *)(base + o_pi);
     X->T.twf = (const uint2 *)(base + o_twf);
     X->T.twi = (const uint2 *)(base + o_twi);
@@ -505,6 +519,10 @@ constexpr int ROWS16_MIN_LOGC = 9;
 static const rows_fn ROWS16[15] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
                                    nullptr, k_rows<9, 4>, k_rows<10, 4>, k_rows<11, 4>, k_rows<12, 4>,
                                    k_rows<13, 4>, k_rows<14, 4>};
+// items of 2^13 words with the tensor-core transforms (rows_tc_kernels.cuh)
+constexpr int ROWS_TC_MIN_LOGC = 9;
+static const rows_fn ROWS_TC[14] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
+                                    k_rows_tc<9>, k_rows_tc<10>, k_rows_tc<11>, k_rows_tc<12>, k_rows_tc<13>};
 #undef FB_COLS
 typedef void (*rows_op_fn)(DevTables, uint32_t *, int, int, int, int);
 static const rows_op_fn ROWS_FWD[15] = {nullptr, nullptr, nullptr, nullptr, nullptr,
@@ -653,6 +671,8 @@ static int configure_kernels()
     }
     for (int c = ROWS16_MIN_LOGC; c <= LOG_MAXC; c++)
         CU(cudaFuncSetAttribute(ROWS16[c], cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    for (int c = ROWS_TC_MIN_LOGC; c < LOG_MAXC; c++)
+        CU(cudaFuncSetAttribute(ROWS_TC[c], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_ROWS_SMEM));
     for (int c = 5; c <= LOG_MAXC; c++) {
         CU(cudaFuncSetAttribute(ROWS[c], cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         CU(cudaFuncSetAttribute(ROWS_FWD[c], cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
@@ -684,6 +704,7 @@ static int ctx_create(Ctx **out, gpu_ulong p)
         cudaError_t e4 = cudaHostAlloc(&X->h_err, sizeof(int), cudaHostAllocDefault);
         if (e1 || e2 || e3 || e4) rc = set_error(GPU_FFT_SMALL_ECUDA, "cudaMalloc of context state failed");
         else {
+            X->T.err = X->d_err;
             cudaMemset(X->d_err, 0, sizeof(int));
             cudaMemset(X->d_ticket, 0, sizeof(unsigned long long));
             *X->h_err = 0;
@@ -959,6 +980,29 @@ static int rows_loge(const Ctx *X, const LaunchShape &L, int np, int ninst)
     return warps < (uint64_t)X->nsm * 16 ? 4 : 5;
 }
 
+// The row pass of ninst products of np primes as one launch: `rows` rows of
+// each prime (stride 2^logR rows), nv rows per item.
+static void launch_rows(const Ctx *X, const LaunchShape &L, int loge, uint32_t *ra, const uint32_t *rb, int logR,
+                        int np, const uint32_t *scale, int squaring, const InstDesc *desc, int ninst, int rows,
+                        cudaStream_t st, bool dep)
+{
+    const int logC = L.S.logC;
+    const int64_t items = (int64_t)((rows + L.nv - 1) / L.nv) * np * ninst;
+    // Items of 2^13 words, which every launch that fills the GPU has, take the
+    // tensor-core kernel (256 uneven products 1199 -> 1071 us, 4096 products mod
+    // 2^47104 + 1 371 -> 353 us, row pass of a 2^24-point product 710 -> 696 us);
+    // 2^14-point rows would need twice its TMEM and shared memory, and launches
+    // short of warps run 16 points per thread.
+    if (loge == 5 && logC >= ROWS_TC_MIN_LOGC && (L.nv << logC) == TC_WORDS && X->T.tcw) {
+        launch_dep(ROWS_TC[logC], (unsigned)std::min<int64_t>(items, 2 * X->nsm), TC_THREADS, TC_ROWS_SMEM, st, dep, X->T,
+                   ra, rb, logR, L.nv, np, scale, squaring, desc, ninst, rows);
+        return;
+    }
+    launch_dep((loge == 4 ? ROWS16 : ROWS)[logC],
+               (unsigned)std::min<int64_t>(items, (int64_t)X->nsm * rows_per_sm(L, loge)), (L.nv << logC) >> loge,
+               L.row_smem, st, dep, X->T, ra, rb, logR, L.nv, np, scale, squaring, desc, ninst, rows);
+}
+
 // The row launch of ninst products of np primes: rows per item as the
 // shape has them (up to 2^13 points per CTA), halved while the launch would
 // have fewer than two items per SM (small transforms).
@@ -1046,8 +1090,7 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
                                                                np, shb, d_scale, fold ? 1 : 0);
         if (early) {
             timing_mark(tr, 1, st);
-            ROWS[S.logC]<<<std::min(L.row_grid * np, X->nsm * rows_per_sm(L)), L.row_threads, L.row_smem, st>>>(
-                X->T, rb, ra, S.logR, L.nv, np, nullptr, 2, nullptr, 1, R);
+            launch_rows(X, L, 5, rb, ra, S.logR, np, nullptr, 2, nullptr, 1, R, st, false);
             timing_mark(tr, 2, st);
             inv<<<dim3(ci.grid, np, 1), ci.threads, ci.smem, st>>>(X->T, rb, S.logC, ci.G, nullptr,
                                                                    ChunkOut{nullptr, 0, 0, 0, 0});
@@ -1061,12 +1104,9 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
     }
     timing_mark(tr, 1, st);
     const LaunchShape Lr = row_launch_shape(X, L, np, ni);
-    const int items = Lr.row_grid * np * ni;
     const int loge = rows_loge(X, Lr, np, ni);
-    launch_dep((loge == 4 ? ROWS16 : ROWS)[S.logC], std::min(items, X->nsm * rows_per_sm(Lr, loge)),
-               (Lr.nv << S.logC) >> loge, Lr.row_smem, st,
-               dep && rows_dependent((size_t)1 << (S.logR + S.logC), S.logC, loge), X->T, ra, rb, S.logR, Lr.nv, np,
-               fold ? nullptr : d_scale, (sq && !desc) ? 1 : 0, desc, ni, R);
+    launch_rows(X, Lr, loge, ra, rb, S.logR, np, fold ? nullptr : d_scale, (sq && !desc) ? 1 : 0, desc, ni, R, st,
+                dep && rows_dependent((size_t)1 << (S.logR + S.logC), S.logC, loge));
     timing_mark(tr, 2, st);
     if (S.logR > 0)
         launch_dep(inv, dim3(ci.grid, np, ni), ci.threads, ci.smem, st, dep && S.logR < 9, X->T, ra, S.logC, ci.G, desc,
@@ -1095,10 +1135,8 @@ static void launch_transforms3(const Ctx *X, int k, int logMs, const uint64_t *a
                X->T, a, an, b, bn, ra, rb, logMs, k, sc, sq ? 0 : 2, fz ? *fz : FzShape{1, 1, 1});
     timing_mark(tr, 1, st);
     const LaunchShape L = make_shape(logMs, LOGC3);   // row launch shape (one 2^13-point row per item)
-    const int items = rows * np;
-    launch_dep(ROWS[LOGC3], std::min(items, X->nsm * rows_per_sm(L)), L.row_threads, L.row_smem, st,
-               rows_dependent((size_t)3 << k, LOGC3), X->T, ra, rb, logMs - LOGC3, 1, np, sq ? sc : nullptr, sq ? 1 : 0,
-               nullptr, 1, rows);
+    launch_rows(X, L, 5, ra, rb, logMs - LOGC3, np, sq ? sc : nullptr, sq ? 1 : 0, nullptr, 1, rows, st,
+                rows_dependent((size_t)3 << k, LOGC3));
     timing_mark(tr, 2, st);
     launch_dep(INV_COLS3[r - LOG3_RMIN], dim3(C / G, np), 512, smem, st, true, X->T, ra, logMs, k);
     timing_mark(tr, 3, st);
@@ -1338,14 +1376,12 @@ static int mpn_mul_enqueue(Ctx *X, uint64_t *z, const uint64_t *a, uint64_t an,
                            Ls.nv * padw(1 << S.logC) * sizeof(uint32_t), st>>>(X->T, cb, S.logR, Ls.nv, np,
                                                                               1 << S.logR);
         launches = 2;
-        const int items = Ls.row_grid * np;
         for (uint64_t i = 0; i * c < xn; i++) {
             const uint64_t xi = std::min(c, xn - i * c);
             const ChunkOut co{ra, logM, i * c, i ? yn - 1 : 0, xi + yn - 1};
             fwd_cols_kernel(S.logR, S.logC)<<<dim3(np, Ls.col_grid, 1), Ls.col_threads, Ls.col_smem, st>>>(
                 X->T, x + i * c, xi, x + i * c, xi, ca, ca, S.logC, S.G, nullptr, np, one, nullptr, 0);
-            ROWS[S.logC]<<<std::min(items, X->nsm * rows_per_sm(Ls)), Ls.row_threads, Ls.row_smem, st>>>(
-                X->T, ca, cb, S.logR, Ls.nv, np, scale_ptr(X, np, Lc), 2, nullptr, 1, 1 << S.logR);
+            launch_rows(X, Ls, 5, ca, cb, S.logR, np, scale_ptr(X, np, Lc), 2, nullptr, 1, 1 << S.logR, st, false);
             inv_cols_kernel(S.logR, S.logC)<<<dim3(Ls.col_grid, np, 1), Ls.col_threads, Ls.col_smem, st>>>(X->T, ca, S.logC, S.G,
                                                                                           nullptr, co);
             launches += 3;

@@ -22,6 +22,7 @@
 // with the serial overhang stitch (mpn_mul.c:802-993, 1934-1973).
 #pragma once
 #include "ntt_smem.cuh"
+#include "tcgen05.cuh"
 
 namespace fb {
 
@@ -53,6 +54,9 @@ struct DevTables {
     const uint2* tw3f;     // [NP3][TW3_SZ] omega^e / 2, omega = w3^(2^14) of order 3 2^11
     const uint2* tw3i;     // [NP3][TW3_SZ] omega^-e / 2
     const uint2* w3c;      // [NP3][2] (w - w^2, w^-1 - w^-2), w = w3^(2^25) of order 3
+    const uint4* tcw;      // [MAX_NP] swizzled W images (tc_fill_w), TC_W_BYTES each
+    const TcPrime* tcp;    // [MAX_NP]
+    int* err;              // the context's device error flag
 };
 
 // Programmatic dependent launch.  A kernel launched as a programmatic
