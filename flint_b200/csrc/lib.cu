@@ -180,6 +180,23 @@ static double log2_product(int np)
     return s;
 }
 
+// the derived CRT constants: 2^(32 np) - P and the quotient's float factors
+static void crt_derive(CrtConst &K)
+{
+    uint64_t c = 1;
+    for (int w = 0; w < K.np; w++) {
+        c += (uint32_t)~K.P[w];
+        K.Pneg[w] = (uint32_t)c;
+        c >>= 32;
+    }
+    double off = 0;
+    for (int j = 0; j < K.np; j++) {
+        K.kc[j] = 256.0f / (float)PRIMES[j];
+        off -= 8388608.0 * (double)K.kc[j];
+    }
+    K.koff = (float)off;
+}
+
 // ---------------------------------------------------------------------------
 // context
 
@@ -380,6 +397,7 @@ static int ctx_build_tables(Ctx *X)
             X->cof_red[np][j] = mw_mod_small(c, PRIMES[j]);
             K.finv[j] = 1.0f / (float)PRIMES[j];
         }
+        crt_derive(K);
     }
 
     size_t off = 0;
@@ -2593,6 +2611,7 @@ static void na_crt_constants(CrtConst &K, uint32_t *cof_red)
         cof_red[j] = (uint32_t)m;
         K.finv[j] = 1.0f / (float)PRIMES[j];
     }
+    crt_derive(K);
 }
 
 // set-up runtime calls: no error message (that would allocate), just the code

@@ -777,6 +777,8 @@ struct CrtConst {
     uint32_t P[MAX_NP];               // product of the primes, 32-bit words
     uint32_t cof[MAX_NP][MAX_NP];     // P / p_j, 32-bit words
     float finv[MAX_NP];
+    uint32_t Pneg[MAX_NP];            // 2^(32 np) - P, np words
+    float kc[MAX_NP], koff;           // 2^8 / p_j; -2^23 sum_j kc[j]
 };
 
 template <int NP>
@@ -800,93 +802,16 @@ __device__ __forceinline__ void crt_coeff(const uint32_t* __restrict__ res, int 
     }
 }
 
-// A[0..5] += y * (c0, c1, c2, c3): one PTX carry chain per partial-product row
-__device__ __forceinline__ void mac4(uint32_t (&A)[7], uint32_t y, const uint32_t* c)
+// (a0 .. a3, a4) += (b0, b1) as 64-bit pairs, with the carry into a4
+__device__ __forceinline__ void add128c(uint32_t (&a)[5], uint64_t b0, uint64_t b1)
 {
-    asm("mad.lo.cc.u32  %0, %7, %8, %0;\n\t"
-        "madc.lo.cc.u32 %1, %7, %9, %1;\n\t"
-        "madc.lo.cc.u32 %2, %7, %10, %2;\n\t"
-        "madc.lo.cc.u32 %3, %7, %11, %3;\n\t"
-        "addc.cc.u32    %4, %4, 0;\n\t"
-        "addc.u32       %5, %5, 0;\n\t"
-        "mad.hi.cc.u32  %1, %7, %8, %1;\n\t"
-        "madc.hi.cc.u32 %2, %7, %9, %2;\n\t"
-        "madc.hi.cc.u32 %3, %7, %10, %3;\n\t"
-        "madc.hi.cc.u32 %4, %7, %11, %4;\n\t"
-        "addc.u32       %5, %5, 0;"
-        : "+r"(A[0]), "+r"(A[1]), "+r"(A[2]), "+r"(A[3]), "+r"(A[4]), "+r"(A[5]), "+r"(A[6])
-        : "r"(y), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]));
-}
-
-// A[0..6] += y * (c0 .. c4)
-__device__ __forceinline__ void mac5(uint32_t (&A)[7], uint32_t y, const uint32_t* c)
-{
-    asm("mad.lo.cc.u32  %0, %7, %8, %0;\n\t"
-        "madc.lo.cc.u32 %1, %7, %9, %1;\n\t"
-        "madc.lo.cc.u32 %2, %7, %10, %2;\n\t"
-        "madc.lo.cc.u32 %3, %7, %11, %3;\n\t"
-        "madc.lo.cc.u32 %4, %7, %12, %4;\n\t"
-        "addc.cc.u32    %5, %5, 0;\n\t"
-        "addc.u32       %6, %6, 0;\n\t"
-        "mad.hi.cc.u32  %1, %7, %8, %1;\n\t"
-        "madc.hi.cc.u32 %2, %7, %9, %2;\n\t"
-        "madc.hi.cc.u32 %3, %7, %10, %3;\n\t"
-        "madc.hi.cc.u32 %4, %7, %11, %4;\n\t"
-        "madc.hi.cc.u32 %5, %7, %12, %5;\n\t"
-        "addc.u32       %6, %6, 0;"
-        : "+r"(A[0]), "+r"(A[1]), "+r"(A[2]), "+r"(A[3]), "+r"(A[4]), "+r"(A[5]), "+r"(A[6])
-        : "r"(y), "r"(c[0]), "r"(c[1]), "r"(c[2]), "r"(c[3]), "r"(c[4]));
-}
-
-// A[0..5] -= k * (P0 .. P4)   (k < 8; the result is non-negative)
-__device__ __forceinline__ void msub5(uint32_t (&A)[7], uint32_t k, const uint32_t* P)
-{
-    asm("{\n\t.reg .u32 t0, t1, t2, t3, t4, t5;\n\t"
-        "mul.lo.u32     t0, %6, %7;\n\t"
-        "mul.lo.u32     t1, %6, %8;\n\t"
-        "mul.lo.u32     t2, %6, %9;\n\t"
-        "mul.lo.u32     t3, %6, %10;\n\t"
-        "mul.lo.u32     t4, %6, %11;\n\t"
-        "mad.hi.cc.u32  t1, %6, %7, t1;\n\t"
-        "madc.hi.cc.u32 t2, %6, %8, t2;\n\t"
-        "madc.hi.cc.u32 t3, %6, %9, t3;\n\t"
-        "madc.hi.cc.u32 t4, %6, %10, t4;\n\t"
-        "madc.hi.u32    t5, %6, %11, 0;\n\t"
-        "sub.cc.u32     %0, %0, t0;\n\t"
-        "subc.cc.u32    %1, %1, t1;\n\t"
-        "subc.cc.u32    %2, %2, t2;\n\t"
-        "subc.cc.u32    %3, %3, t3;\n\t"
-        "subc.cc.u32    %4, %4, t4;\n\t"
-        "subc.u32       %5, %5, t5;\n\t}"
-        : "+r"(A[0]), "+r"(A[1]), "+r"(A[2]), "+r"(A[3]), "+r"(A[4]), "+r"(A[5])
-        : "r"(k), "r"(P[0]), "r"(P[1]), "r"(P[2]), "r"(P[3]), "r"(P[4]));
-}
-
-// A[0..6] -= k * (P0 .. P5)
-__device__ __forceinline__ void msub6(uint32_t (&A)[7], uint32_t k, const uint32_t* P)
-{
-    asm("{\n\t.reg .u32 t0, t1, t2, t3, t4, t5, t6;\n\t"
-        "mul.lo.u32     t0, %7, %8;\n\t"
-        "mul.lo.u32     t1, %7, %9;\n\t"
-        "mul.lo.u32     t2, %7, %10;\n\t"
-        "mul.lo.u32     t3, %7, %11;\n\t"
-        "mul.lo.u32     t4, %7, %12;\n\t"
-        "mul.lo.u32     t5, %7, %13;\n\t"
-        "mad.hi.cc.u32  t1, %7, %8, t1;\n\t"
-        "madc.hi.cc.u32 t2, %7, %9, t2;\n\t"
-        "madc.hi.cc.u32 t3, %7, %10, t3;\n\t"
-        "madc.hi.cc.u32 t4, %7, %11, t4;\n\t"
-        "madc.hi.cc.u32 t5, %7, %12, t5;\n\t"
-        "madc.hi.u32    t6, %7, %13, 0;\n\t"
-        "sub.cc.u32     %0, %0, t0;\n\t"
-        "subc.cc.u32    %1, %1, t1;\n\t"
-        "subc.cc.u32    %2, %2, t2;\n\t"
-        "subc.cc.u32    %3, %3, t3;\n\t"
-        "subc.cc.u32    %4, %4, t4;\n\t"
-        "subc.cc.u32    %5, %5, t5;\n\t"
-        "subc.u32       %6, %6, t6;\n\t}"
-        : "+r"(A[0]), "+r"(A[1]), "+r"(A[2]), "+r"(A[3]), "+r"(A[4]), "+r"(A[5]), "+r"(A[6])
-        : "r"(k), "r"(P[0]), "r"(P[1]), "r"(P[2]), "r"(P[3]), "r"(P[4]), "r"(P[5]));
+    asm("add.cc.u32  %0, %0, %5;\n\t"
+        "addc.cc.u32 %1, %1, %6;\n\t"
+        "addc.cc.u32 %2, %2, %7;\n\t"
+        "addc.cc.u32 %3, %3, %8;\n\t"
+        "addc.u32    %4, %4, 0;"
+        : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4])
+        : "r"((uint32_t)b0), "r"((uint32_t)(b0 >> 32)), "r"((uint32_t)b1), "r"((uint32_t)(b1 >> 32)));
 }
 
 template <int NP>
@@ -894,22 +819,64 @@ __device__ __forceinline__ void crt_values(const uint32_t (&y)[NP], const CrtCon
                                            uint64_t& c1, uint64_t& c2)
 {
     if constexpr (NP == 5 || NP == 6) {
-        // carry-chain form: X = sum_j y_j (P/p_j) - k P in 32-bit words
-        float fk = 0.0f;
+        // X = sum_j y_j (P/p_j) - k P modulo 2^(32 NP), as 64-bit products of
+        // 32-bit words summed without carries: y_j c < p_j 2^32, and the pairs
+        // (0, 1), (2, 3) and (4, 5) of primes sum to less than 2^32 each, with
+        // room for k (2^(32 NP) - P), k < 8, beside the last.  (One 64-bit
+        // product-sum holds the FMA pipe for 4.3 cycles a warp where the low and
+        // high halves by themselves take 6.)
+        // k = round(sum_j y_j / p_j) from the top 23 bits of each y_j under the
+        // exponent of 2^23: no integer-to-float conversions; off by less than
+        // 10^-5, and the coefficient bound leaves 3 10^-4.
+        float fk = K.koff;
 #pragma unroll
-        for (int jp = 0; jp < NP; jp++) fk = fmaf((float)y[jp], K.finv[jp], fk);
-        uint32_t A[7] = {0, 0, 0, 0, 0, 0, 0};
+        for (int jp = 0; jp < NP; jp++)
+            fk = fmaf(__uint_as_float(__byte_perm(y[jp], 0x4bu, 0x4321)), K.kc[jp], fk);
+        const uint32_t k = __float_as_uint(fk + 12582912.0f) & 0xffu;   // 1.5 2^23: rounds to an integer
+        constexpr int CW = NP - 1;
+        uint64_t g[3][CW];
 #pragma unroll
-        for (int jp = 0; jp < NP; jp++) {
-            if constexpr (NP == 5) mac4(A, y[jp], K.cof[jp]);
-            else mac5(A, y[jp], K.cof[jp]);
+        for (int w = 0; w < CW; w++) {
+            g[0][w] = (uint64_t)y[0] * K.cof[0][w] + (uint64_t)y[1] * K.cof[1][w];
+            g[1][w] = (uint64_t)y[2] * K.cof[2][w] + (uint64_t)y[3] * K.cof[3][w];
+            g[2][w] = (uint64_t)y[4] * K.cof[4][w] + (uint64_t)k * K.Pneg[w];
+            if constexpr (NP == 6) g[2][w] += (uint64_t)y[5] * K.cof[5][w];
         }
-        const uint32_t k = (uint32_t)rintf(fk);
-        if constexpr (NP == 5) msub5(A, k, K.P);
-        else msub6(A, k, K.P);
-        c0 = (uint64_t)A[0] | ((uint64_t)A[1] << 32);
-        c1 = (uint64_t)A[2] | ((uint64_t)A[3] << 32);
-        c2 = (uint64_t)A[4] | (NP == 6 ? ((uint64_t)A[5] << 32) : 0ull);
+        // even words e (0 .. 3, carries into word 4), odd words o (1 .. 4, and
+        // 5 for six primes)
+        uint32_t e[5] = {(uint32_t)g[0][0], (uint32_t)(g[0][0] >> 32), (uint32_t)g[0][2], (uint32_t)(g[0][2] >> 32), 0};
+        uint32_t o[5] = {(uint32_t)g[0][1], (uint32_t)(g[0][1] >> 32), (uint32_t)g[0][3], (uint32_t)(g[0][3] >> 32), 0};
+#pragma unroll
+        for (int t = 1; t < 3; t++) {
+            add128c(e, g[t][0], g[t][2]);
+            add128c(o, g[t][1], g[t][3]);
+        }
+        if constexpr (NP == 5) {
+            e[4] += k * K.Pneg[4];
+            asm("add.cc.u32  %0, %0, %4;\n\t"
+                "addc.cc.u32 %1, %1, %5;\n\t"
+                "addc.cc.u32 %2, %2, %6;\n\t"
+                "addc.u32    %3, %3, %7;"
+                : "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(e[4])
+                : "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]));
+            c2 = (uint64_t)e[4];
+        } else {
+            // words 4, 5: the products at word 4, the carries out of the even and
+            // odd words below, and k Pneg at word 5
+            const uint64_t top = g[0][4] + g[1][4] + g[2][4] + e[4] + ((uint64_t)(k * K.Pneg[5]) << 32) +
+                                 ((uint64_t)o[4] << 32);
+            uint32_t t4 = (uint32_t)top, t5 = (uint32_t)(top >> 32);
+            asm("add.cc.u32  %0, %0, %5;\n\t"
+                "addc.cc.u32 %1, %1, %6;\n\t"
+                "addc.cc.u32 %2, %2, %7;\n\t"
+                "addc.cc.u32 %3, %3, %8;\n\t"
+                "addc.u32    %4, %4, 0;"
+                : "+r"(e[1]), "+r"(e[2]), "+r"(e[3]), "+r"(t4), "+r"(t5)
+                : "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]));
+            c2 = (uint64_t)t4 | ((uint64_t)t5 << 32);
+        }
+        c0 = (uint64_t)e[0] | ((uint64_t)e[1] << 32);
+        c1 = (uint64_t)e[2] | ((uint64_t)e[3] << 32);
         return;
     }
     float fk = 0.0f;
@@ -962,7 +929,10 @@ constexpr long LOOKBACK_SPIN_LIMIT = 1L << 22;
 // Residue CRT/carry tiles: CRT_THREADS threads of 4 coefficients.  Measured
 // on the B200 (2^24 x 2^24 product): 128-thread tiles 0.330 ms, 256 0.337,
 // 512 0.377 -- smaller tiles keep more of them resident per SM while one
-// waits on its ticket or look-back.
+// waits on its ticket or look-back.  The recombination is what bounds them: with
+// 64-bit product-sums (crt_values) 0.330 -> 0.289 ms, against 0.144 ms of HBM
+// traffic; persistent CTAs that draw the next ticket and load its residues ahead
+// were slower (0.349 ms: 72 registers and fewer CTAs per SM).
 constexpr int CRT_THREADS = 128;
 constexpr int CRT_TILE = 4 * CRT_THREADS;
 
