@@ -552,6 +552,17 @@ static const rows_op_fn ROWS_INV[15] = {nullptr, nullptr, nullptr, nullptr, null
                                         k_rows_inv<9>, k_rows_inv<10>, k_rows_inv<11>, k_rows_inv<12>,
                                         k_rows_inv<13>, k_rows_inv<14>};
 
+// one-row transforms in one launch (index logC - 9, [16 words per thread],
+// [polynomial operands])
+typedef void (*rows_small_fn)(DevTables, const uint64_t *, uint64_t, const uint64_t *, uint64_t, uint32_t *,
+                              const uint32_t *, int, const InstDesc *, FzShape);
+constexpr int SMALL_MIN_LOGC = 9, SMALL_MAX_LOGC = 12;
+static const rows_small_fn ROWS_SMALL[4][2][2] = {
+    {{k_rows_small<9, false, 3>, k_rows_small<9, true, 3>}, {k_rows_small<9, false, 4>, k_rows_small<9, true, 4>}},
+    {{k_rows_small<10, false, 3>, k_rows_small<10, true, 3>}, {k_rows_small<10, false, 4>, k_rows_small<10, true, 4>}},
+    {{k_rows_small<11, false, 3>, k_rows_small<11, true, 3>}, {k_rows_small<11, false, 4>, k_rows_small<11, true, 4>}},
+    {{k_rows_small<12, false, 3>, k_rows_small<12, true, 3>}, {k_rows_small<12, false, 4>, k_rows_small<12, true, 4>}}};
+
 constexpr int MIN_LOGM = 5;
 
 struct LaunchShape {
@@ -564,21 +575,49 @@ struct LaunchShape {
 };
 
 // Four-step split of a 2^logM transform: rows of 2^logC, columns of
-// 2^(logM - logC); logC < 0 takes the longest rows (2^14), which leaves the
-// shortest columns.
+// 2^(logM - logC); logC < 0 takes single_logC's.
 constexpr int LOG_MAXR = 11;
-// Default row length: the whole transform up to 2^13 points; 2^5-point
-// columns from 2^14 to 2^17 points and 2^6 at 2^18 (small transforms are
-// latency-bound, and 32-point columns spread a product over the most CTAs:
-// measured 2^15-point products 0.056 -> 0.030 ms, 2^17-point 0.062 -> 0.038
-// ms); 2^13-point rows from 2^19 to 2^24 (more row items for mid sizes), 2^14
-// at 2^25 where the columns reach their longest length.
+// Row length of a configuration that leaves it open: the whole transform up to
+// 2^13 points, 2^5-point columns from 2^14 to 2^17 and 2^6 at 2^18, 2^13-point rows
+// from 2^19 to 2^24, 2^14 at 2^25.
 static int default_logC(int logM)
 {
     if (logM <= LOG_MAXC - 1) return logM;
     if (logM <= 17) return logM - 5;
     if (logM == 18) return 12;
     return std::max(LOG_MAXC - 1, logM - LOG_MAXR);
+}
+// Row length without a configuration: the whole transform up to 2^12 points (one launch);
+// 4-point columns at 2^13 and 2^14 and 2^5-point ones from 2^15 to 2^17, 2^6 at
+// 2^18 (small transforms are latency-bound: what counts is how few instructions
+// the row pass's warps run and over how many SMs); 2^11-point rows at 2^19 and
+// 2^12 at 2^20 (one strided pass fewer than 2^13, enough columns), 2^13 from 2^21
+// to 2^24, 2^14 at 2^25 where the columns reach their longest length.  Measured,
+// n x n limbs, us by log2 of the row length: 2^13 points 11: 15.4, 12: 15.5, 13:
+// 19.9; 2^14 12: 17.8, 11: 18.8, 9: 21.3; 2^15 12: 21.3, 10: 21.6; 2^16 11: 23.0,
+// 10: 26.4; 2^17 12: 29.4, 11: 30.4; 2^18 12: 42.0, 10: 43.0; 2^19 11: 73.8, 12:
+// 75.9, 13: 77.9; 2^20 12: 118.6, 11: 119.8, 13: 122.1; 2^21 12: 219.3, 13: 219.7;
+// 2^22 13: 422.5, 11: 439.5.
+static int single_logC(int logM)
+{
+    if (logM <= 12) return logM;
+    if (logM <= 14) return logM - 2;
+    if (logM <= 17) return logM - 5;
+    if (logM == 18) return 12;
+    if (logM <= 20) return logM - 8;
+    return std::max(LOG_MAXC - 1, logM - LOG_MAXR);
+}
+// Row length of a planned batch's class, whose launches fill the GPU whatever
+// the shape: whole rows up to 2^13 points, then rows of 2^9 (one strided pass
+// before the tensor cores), 2^11 at 2^19.  Measured, us a product in a batch of
+// equal ones: 2^13 points 13: 0.80, 11: 0.88; 2^14 9: 1.29, 5: 1.44, 12 above
+// 1.64; 2^15 9: 2.80, 10: 2.83; 2^16 9: 5.62, 11: 5.65; 2^17 9: 11.31, 12: 11.89;
+// 2^18 9: 23.4, 12: 25.7; 2^19 11: 49.4, 13: 53.7.
+static int batch_logC(int logM)
+{
+    if (logM <= 13) return logM;
+    if (logM <= 18) return 9;
+    return logM == 19 ? 11 : single_logC(logM);
 }
 // Shortest row for a transform of 2^logM points: columns at most 2^11 long,
 // and with 32 or more columns (the column kernel's 2^14-word tiles of
@@ -598,7 +637,7 @@ static bool valid_logC(int logM, int logC)
 static LaunchShape make_shape(int logM, int logC = -1)
 {
     LaunchShape L;
-    L.S.logC = logC < 0 ? default_logC(logM) : logC;
+    L.S.logC = logC < 0 ? single_logC(logM) : logC;
     L.S.logR = logM - L.S.logC;
     const int R = 1 << L.S.logR, C = 1 << L.S.logC;
     if (L.S.logR >= 5) {
@@ -647,7 +686,7 @@ static void launch_dep(void (*f)(P...), dim3 grid, dim3 block, size_t smem, cuda
 // compiled in (rows_dep) and never runs as one.
 static bool rows_dependent(size_t points, int logC, int loge = 5)
 {
-    return points <= (size_t)1 << 20 && (logC < LOG_MAXC || loge == 4);
+    return points <= (size_t)1 << 20 && (logC < LOG_MAXC || loge < 5);
 }
 
 // the three transform launches shared by every product type; with a batch
@@ -969,16 +1008,18 @@ static int upload_scales(Ctx *X)
     return 0;
 }
 
+static rows_fn rows_kernel(int logC, int loge) { return (loge == 4 ? ROWS16 : ROWS)[logC]; }
+
 // Resident row CTAs per SM for a shape: 1 for long rows (512 threads, ~135 KB
 // of shared memory), several for short ones.  The row launch depends on the
 // row length and the rows per item.
 static int rows_per_sm(const LaunchShape &L, int loge = 5)
 {
     static int occ[2][LOG_MAXC + 1][LOG_MAXC + 1] = {{{0}}};
-    const int c = L.S.logC, v = __builtin_ctz((unsigned)L.nv), e = loge == 4;
+    const int c = L.S.logC, v = __builtin_ctz((unsigned)L.nv), e = 5 - loge;
     if (occ[e][c][v] == 0) {
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, e ? ROWS16[c] : ROWS[c], (L.nv << c) >> loge,
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rows_kernel(c, loge), (L.nv << c) >> loge,
                                                           L.row_smem) != cudaSuccess || n < 1)
             n = 1;
         occ[e][c][v] = n;
@@ -1016,7 +1057,7 @@ static void launch_rows(const Ctx *X, const LaunchShape &L, int loge, uint32_t *
                    ra, rb, logR, L.nv, np, scale, squaring, desc, ninst, rows);
         return;
     }
-    launch_dep((loge == 4 ? ROWS16 : ROWS)[logC],
+    launch_dep(rows_kernel(logC, loge),
                (unsigned)std::min<int64_t>(items, (int64_t)X->nsm * rows_per_sm(L, loge)), (L.nv << logC) >> loge,
                L.row_smem, st, dep, X->T, ra, rb, logR, L.nv, np, scale, squaring, desc, ninst, rows);
 }
@@ -1087,6 +1128,18 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
     // a batch's launches are the nodes of its graph, without launch gaps
     const bool dep = !desc;
     const int R = 1 << S.logR;
+    if (S.logR == 0 && S.logC >= SMALL_MIN_LOGC && S.logC <= SMALL_MAX_LOGC && !L.loge && !co) {
+        if (b_ready) cudaStreamWaitEvent(st, b_ready, 0);
+        timing_mark(tr, 1, st);
+        // eight words per thread until sixteen would fill the SMs with 8 warps
+        const int w16 = ((int64_t)np * ni << S.logC) >> 9 >= (int64_t)X->nsm * 8;
+        launch_dep(ROWS_SMALL[S.logC - SMALL_MIN_LOGC][w16][fz != nullptr], dim3(np, ni), (1 << S.logC) >> (3 + w16),
+                   2 * padw(1 << S.logC) * sizeof(uint32_t), st, !desc && !b_ready, X->T, a, an, b, bn, ra, d_scale,
+                   (sq && !desc) ? 1 : 0, desc, shape);
+        timing_mark(tr, 2, st);
+        timing_mark(tr, 3, st);
+        return ra;
+    }
     if (b_ready && !desc && !sq) {
         // b is still arriving: a's column pass first, b's after its copy
         fwd<<<dim3(np, cf.grid, 1), cf.threads, cf.smem, st>>>(X->T, a, an, a, an, ra, ra, S.logC, cf.G, nullptr,

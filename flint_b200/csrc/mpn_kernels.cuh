@@ -502,10 +502,10 @@ __device__ __forceinline__ void rows_prefetch(uint32_t* dst, const uint32_t* __r
 // 2^14-point rows at 32 points per thread run large products only, which gain
 // nothing from an early launch (1.474 ms; 1.483 ms with the wait compiled in).
 template <int LOGC, int LOGE>
-__device__ __host__ constexpr bool rows_dep() { return LOGC < LOG_MAXC || LOGE == 4; }
+__device__ __host__ constexpr bool rows_dep() { return LOGC < LOG_MAXC || LOGE < 5; }
 
 template <int LOGC, int LOGE = 5>
-__global__ void __launch_bounds__(LOGE == 4 ? 1024 : 512, 1)
+__global__ void __launch_bounds__(LOGE < 5 ? 1024 : 512, 1)
 k_rows(DevTables T, uint32_t* __restrict__ ra, const uint32_t* __restrict__ rb,
        int logR, int nv, int np, const uint32_t* __restrict__ scale, int squaring,
        const InstDesc* __restrict__ desc, int ninst, int rows)
@@ -655,6 +655,88 @@ k_rows(DevTables T, uint32_t* __restrict__ ra, const uint32_t* __restrict__ rb,
         cur ^= 1;
     }
     cp_async_wait<0>();
+}
+
+// ---------------------------------------------------------------------------
+// Transforms of one row (M = 2^LOGC points, no columns) in one launch: split,
+// forward transforms of a and b, pointwise product, inverse transform.  One CTA
+// per (prime, product), C / 2^LOGE threads; grid = (np, instances), smem =
+// 2 padw(C) words; arguments as k_fwd_cols and k_rows.  A product of this
+// length is bound by latency: launches, and instructions that every warp runs
+// once from a cold cache.  Eight words per thread halve a warp's instructions
+// against sixteen (256 x 256 limbs: 10.4 us with the split as a launch of its own,
+// 11.4 us here with sixteen words per thread, 7.9 us with eight; 2048 x 2048:
+// 13.2, 15.7, 13.0); a batch with enough products is bound by their number and
+// takes sixteen (2^11 points 0.31 us a product with the split apart, 0.16 here,
+// 0.18 with eight).
+template <int LOGC, bool FZ, int LOGE>
+__global__ void __launch_bounds__(1 << (LOGC - LOGE))
+k_rows_small(DevTables T, const uint64_t* __restrict__ a, uint64_t an, const uint64_t* __restrict__ b, uint64_t bn,
+             uint32_t* __restrict__ ra, const uint32_t* __restrict__ scale, int squaring,
+             const InstDesc* __restrict__ desc, FzShape fz)
+{
+    extern __shared__ uint32_t sm[];
+    constexpr int C = 1 << LOGC, E = 1 << LOGE, NT = C / E;
+    static_assert(NT % 32 == 0, "whole warps");
+    const int t = threadIdx.x, j = blockIdx.x;
+    pdl_wait();
+    pdl_trigger();
+    if (desc) {
+        const InstDesc& D = desc[blockIdx.y];
+        a = D.a; b = D.b; an = D.an; bn = D.bn;
+        ra = D.ra;
+    }
+    const PrimeInfo P = T.pi[j];
+    const uint32_t p = P.p;
+    uint32_t* const sa = sm;
+    uint32_t* const sb = sm + padw(C);
+    auto split = [&](uint32_t* s, const uint64_t* __restrict__ x, uint64_t xn, uint32_t xw) {
+        if (FZ || xn <= (uint64_t)C) {
+#pragma unroll
+            for (int k = 0; k < E; k++)
+                s[padw(t) + k * (NT / 32 * 33)] = load_residue<FZ>(x, (uint64_t)(t + k * NT), xn, fz.S, xw, P);
+        } else {
+            // an operand longer than the transform wraps around (x mod X^C - 1)
+            for (int k = 0; k < E; k++) {
+                uint32_t r = 0;
+                for (uint64_t n = (uint64_t)(t + k * NT); n < xn; n += C)
+                    r = add_mod(r, limb_redc(x[n], p, P.pneg_inv, P.c32), p);
+                s[padw(t) + k * (NT / 32 * 33)] = r;
+            }
+        }
+    };
+    split(sa, a, an, fz.wa);
+    if (!squaring) split(sb, b, bn, fz.wb);
+    __syncthreads();
+    const uint2* __restrict__ twf = T.twf + (size_t)j * TW_SZ;
+    const uint2* __restrict__ twi = T.twi + (size_t)j * TW_SZ;
+    const int pb = padw(E * t);
+    uint32_t xr[E], br[E];
+    if (!squaring) {
+        gs_strided_all2<LOGC, LOGE, LOGE>(sa, sb, 1, twf, p);
+#pragma unroll
+        for (int m = 0; m < E; m++) {
+            xr[m] = sa[pb + m];
+            br[m] = sb[pb + m];
+        }
+        gs_contig2<LOGE, ROW_GS_FMA_ADDS>(xr, br, c_w32[j], p);
+    } else {
+        gs_strided_all<LOGC, 0, LOGE, LOGE>(sa, 1, twf, p);
+#pragma unroll
+        for (int m = 0; m < E; m++) xr[m] = sa[pb + m];
+        gs_contig<LOGE, ROW_GS_FMA_ADDS>(xr, c_w32[j], p);
+    }
+    const uint32_t sc = scale[j];
+#pragma unroll
+    for (int m = 0; m < E; m++) {
+        const uint32_t y = squaring ? xr[m] : br[m];
+        xr[m] = mul_mont(mul_mont(xr[m], y, p, P.pneg_inv), sc, p, P.pneg_inv);
+    }
+    ct_contig<LOGE, ROW_CT_FMA_ADDS>(xr, c_w32[j], p);
+#pragma unroll
+    for (int m = 0; m < E; m++) sa[pb + m] = xr[m];
+    __syncthreads();
+    ct_strided_all_out<LOGC, LOGE, LOGE>(sa, twi, p, ra + ((size_t)j << LOGC));
 }
 
 // Destination of one chunk of a split product (a long operand cut into

@@ -248,9 +248,10 @@ __device__ __forceinline__ void gs_pass_smem(uint32_t* sm, int nv, const uint2* 
     constexpr int NSUB = L / E;
     const int TOT = (G ? G : nv) * NSUB;
     // element m of a sub-transform sits at pb + padw(m S G'): a compile-time
-    // offset when S G' is a multiple of 32, and also for S = 16 in the rows
-    // layout (the base then lies in the low half of a 32-word bank row)
-    static_assert(S * (G ? G : 1) % 32 == 0 || (G == 0 && S == 16), "unsupported pass stride");
+    // offset when S G' is a multiple of 32, and also for S = 16 and S = 8 in the
+    // rows layout (the base is below S modulo 16 or 32, so adding m S carries
+    // into the next 32-word bank row exactly when m S does)
+    static_assert(S * (G ? G : 1) % 32 == 0 || (G == 0 && (S == 16 || S == 8)), "unsupported pass stride");
     constexpr int SG = S * (G ? G : 1);
 #pragma unroll PASS_UNROLL
     for (int f = threadIdx.x; f < TOT; f += blockDim.x) {
@@ -279,7 +280,7 @@ __device__ __forceinline__ void gs_pass_smem2(uint32_t* sx, uint32_t* sy, int nv
     constexpr int S = H >> (Q - 1);
     constexpr int NSUB = L / E;
     const int TOT = nv * NSUB;
-    static_assert(S % 32 == 0 || S == 16, "unsupported pass stride");
+    static_assert(S % 32 == 0 || S == 16 || S == 8, "unsupported pass stride");
 #pragma unroll PASS_UNROLL
     for (int f = threadIdx.x; f < TOT; f += blockDim.x) {
         const int s = f & (NSUB - 1), v = f / NSUB;
@@ -309,7 +310,7 @@ __device__ __forceinline__ void ct_pass_smem(uint32_t* sm, int nv, const uint2* 
     constexpr int S = H;
     constexpr int NSUB = L / E;
     const int TOT = (G ? G : nv) * NSUB;
-    static_assert(S * (G ? G : 1) % 32 == 0 || (G == 0 && S == 16), "unsupported pass stride");
+    static_assert(S * (G ? G : 1) % 32 == 0 || (G == 0 && (S == 16 || S == 8)), "unsupported pass stride");
     constexpr int SG = S * (G ? G : 1);
 #pragma unroll PASS_UNROLL
     for (int f = threadIdx.x; f < TOT; f += blockDim.x) {
