@@ -279,7 +279,21 @@ static int timing_scratch(Ctx *X, size_t bytes, uint64_t **buf)
     return 0;
 }
 
-static int ctx_build_tables(Ctx *X)
+// Every table a context uploads, which depend on the prime set alone: built by
+// the process's first context and kept (about 5 MB), as one image of the device
+// tables with its offsets, the pointwise scales and the CRT constants.
+struct HostTables {
+    std::vector<char> image;
+    size_t o_pi, o_twf, o_twi, o_th, o_tl, o_thi, o_tli, o_th3, o_tl3, o_th3i, o_tl3i, o_tw3f, o_tw3i, o_w3c, o_tcw, o_tcp;
+    std::vector<uint32_t> scales;
+    CrtConst crt[MAX_NP + 1];
+    uint32_t cof_red[MAX_NP + 1][MAX_NP];
+    HostTables();
+};
+
+static void fill_scales(HostTables &H);
+
+HostTables::HostTables()
 {
     const size_t n_twf = (size_t)MAX_NP * TW_SZ;
     const size_t n_th = (size_t)MAX_NP * TH_SZ;
@@ -385,7 +399,7 @@ static int ctx_build_tables(Ctx *X)
     }
     // CRT constants for every prime count
     for (int np = 1; np <= MAX_NP; np++) {
-        CrtConst &K = X->crt[np];
+        CrtConst &K = crt[np];
         memset(&K, 0, sizeof K);
         K.np = np;
         std::vector<uint32_t> P = {1};
@@ -394,7 +408,7 @@ static int ctx_build_tables(Ctx *X)
         for (int j = 0; j < np; j++) {
             std::vector<uint32_t> c = mw_div_small(P, PRIMES[j]);
             for (size_t w = 0; w < c.size() && w < (size_t)MAX_NP; w++) K.cof[j][w] = c[w];
-            X->cof_red[np][j] = mw_mod_small(c, PRIMES[j]);
+            cof_red[np][j] = mw_mod_small(c, PRIMES[j]);
             K.finv[j] = 1.0f / (float)PRIMES[j];
         }
         crt_derive(K);
@@ -402,49 +416,65 @@ static int ctx_build_tables(Ctx *X)
 
     size_t off = 0;
     auto place = [&](size_t bytes) { size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
-    const size_t o_pi = place(sizeof(PrimeInfo) * MAX_NP);
-    const size_t o_twf = place(sizeof(uint2) * n_twf), o_twi = place(sizeof(uint2) * n_twf);
-    const size_t o_th = place(sizeof(uint2) * n_th), o_tl = place(sizeof(uint2) * n_tl);
-    const size_t o_thi = place(sizeof(uint2) * n_th), o_tli = place(sizeof(uint2) * n_tl);
-    const size_t o_th3 = place(sizeof(uint2) * n_th3), o_tl3 = place(sizeof(uint2) * n_tl3);
-    const size_t o_th3i = place(sizeof(uint2) * n_th3), o_tl3i = place(sizeof(uint2) * n_tl3);
-    const size_t o_tw3f = place(sizeof(uint2) * n_tw3), o_tw3i = place(sizeof(uint2) * n_tw3);
-    const size_t o_w3c = place(sizeof(uint2) * NP3 * 2);
-    const size_t o_tcw = place((size_t)TC_W_BYTES * MAX_NP), o_tcp = place(sizeof(TcPrime) * MAX_NP);
-    CU(cudaMalloc(&X->d_tables, off));
-    char *base = (char *)X->d_tables;
-    CU(cudaMemcpy(base + o_pi, pi.data(), sizeof(PrimeInfo) * MAX_NP, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_twf, twf.data(), sizeof(uint2) * n_twf, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_twi, twi.data(), sizeof(uint2) * n_twf, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_th, th.data(), sizeof(uint2) * n_th, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_tl, tl.data(), sizeof(uint2) * n_tl, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_thi, thi.data(), sizeof(uint2) * n_th, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_tli, tli.data(), sizeof(uint2) * n_tl, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_th3, th3.data(), sizeof(uint2) * n_th3, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_tl3, tl3.data(), sizeof(uint2) * n_tl3, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_th3i, th3i.data(), sizeof(uint2) * n_th3, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_tl3i, tl3i.data(), sizeof(uint2) * n_tl3, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_tw3f, tw3f.data(), sizeof(uint2) * n_tw3, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_tw3i, tw3i.data(), sizeof(uint2) * n_tw3, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_w3c, w3c.data(), sizeof(uint2) * NP3 * 2, cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_tcw, tcw.data(), tcw.size(), cudaMemcpyHostToDevice));
-    CU(cudaMemcpy(base + o_tcp, tcp.data(), sizeof(TcPrime) * MAX_NP, cudaMemcpyHostToDevice));
-    X->T.tcw = (const uint4 *)(base + o_tcw);
-    X->T.tcp = (const TcPrime *)(base + o_tcp);
-    X->T.pi = (const PrimeInfo *)(base + o_pi);
-    X->T.twf = (const uint2 *)(base + o_twf);
-    X->T.twi = (const uint2 *)(base + o_twi);
-    X->T.th = (const uint2 *)(base + o_th);
-    X->T.tl = (const uint2 *)(base + o_tl);
-    X->T.thi = (const uint2 *)(base + o_thi);
-    X->T.tli = (const uint2 *)(base + o_tli);
-    X->T.th3 = (const uint2 *)(base + o_th3);
-    X->T.tl3 = (const uint2 *)(base + o_tl3);
-    X->T.th3i = (const uint2 *)(base + o_th3i);
-    X->T.tl3i = (const uint2 *)(base + o_tl3i);
-    X->T.tw3f = (const uint2 *)(base + o_tw3f);
-    X->T.tw3i = (const uint2 *)(base + o_tw3i);
-    X->T.w3c = (const uint2 *)(base + o_w3c);
+    o_pi = place(sizeof(PrimeInfo) * MAX_NP);
+    o_twf = place(sizeof(uint2) * n_twf); o_twi = place(sizeof(uint2) * n_twf);
+    o_th = place(sizeof(uint2) * n_th); o_tl = place(sizeof(uint2) * n_tl);
+    o_thi = place(sizeof(uint2) * n_th); o_tli = place(sizeof(uint2) * n_tl);
+    o_th3 = place(sizeof(uint2) * n_th3); o_tl3 = place(sizeof(uint2) * n_tl3);
+    o_th3i = place(sizeof(uint2) * n_th3); o_tl3i = place(sizeof(uint2) * n_tl3);
+    o_tw3f = place(sizeof(uint2) * n_tw3); o_tw3i = place(sizeof(uint2) * n_tw3);
+    o_w3c = place(sizeof(uint2) * NP3 * 2);
+    o_tcw = place((size_t)TC_W_BYTES * MAX_NP); o_tcp = place(sizeof(TcPrime) * MAX_NP);
+    image.resize(off);
+    memcpy(&image[o_pi], pi.data(), sizeof(PrimeInfo) * MAX_NP);
+    memcpy(&image[o_twf], twf.data(), sizeof(uint2) * n_twf);
+    memcpy(&image[o_twi], twi.data(), sizeof(uint2) * n_twf);
+    memcpy(&image[o_th], th.data(), sizeof(uint2) * n_th);
+    memcpy(&image[o_tl], tl.data(), sizeof(uint2) * n_tl);
+    memcpy(&image[o_thi], thi.data(), sizeof(uint2) * n_th);
+    memcpy(&image[o_tli], tli.data(), sizeof(uint2) * n_tl);
+    memcpy(&image[o_th3], th3.data(), sizeof(uint2) * n_th3);
+    memcpy(&image[o_tl3], tl3.data(), sizeof(uint2) * n_tl3);
+    memcpy(&image[o_th3i], th3i.data(), sizeof(uint2) * n_th3);
+    memcpy(&image[o_tl3i], tl3i.data(), sizeof(uint2) * n_tl3);
+    memcpy(&image[o_tw3f], tw3f.data(), sizeof(uint2) * n_tw3);
+    memcpy(&image[o_tw3i], tw3i.data(), sizeof(uint2) * n_tw3);
+    memcpy(&image[o_w3c], w3c.data(), sizeof(uint2) * NP3 * 2);
+    memcpy(&image[o_tcw], tcw.data(), tcw.size());
+    memcpy(&image[o_tcp], tcp.data(), sizeof(TcPrime) * MAX_NP);
+    fill_scales(*this);
+}
+
+static const HostTables &host_tables()
+{
+    static const HostTables H;
+    return H;
+}
+
+static int ctx_build_tables(Ctx *X)
+{
+    const HostTables &H = host_tables();
+    memcpy(X->crt, H.crt, sizeof H.crt);
+    memcpy(X->cof_red, H.cof_red, sizeof H.cof_red);
+    CU(cudaMalloc(&X->d_tables, H.image.size()));
+    CU(cudaMemcpy(X->d_tables, H.image.data(), H.image.size(), cudaMemcpyHostToDevice));
+    const char *base = (const char *)X->d_tables;
+    X->T.tcw = (const uint4 *)(base + H.o_tcw);
+    X->T.tcp = (const TcPrime *)(base + H.o_tcp);
+    X->T.pi = (const PrimeInfo *)(base + H.o_pi);
+    X->T.twf = (const uint2 *)(base + H.o_twf);
+    X->T.twi = (const uint2 *)(base + H.o_twi);
+    X->T.th = (const uint2 *)(base + H.o_th);
+    X->T.tl = (const uint2 *)(base + H.o_tl);
+    X->T.thi = (const uint2 *)(base + H.o_thi);
+    X->T.tli = (const uint2 *)(base + H.o_tli);
+    X->T.th3 = (const uint2 *)(base + H.o_th3);
+    X->T.tl3 = (const uint2 *)(base + H.o_tl3);
+    X->T.th3i = (const uint2 *)(base + H.o_th3i);
+    X->T.tl3i = (const uint2 *)(base + H.o_tl3i);
+    X->T.tw3f = (const uint2 *)(base + H.o_tw3f);
+    X->T.tw3i = (const uint2 *)(base + H.o_tw3i);
+    X->T.w3c = (const uint2 *)(base + H.o_w3c);
     // constant memory belongs to the current device's module instance
     CU(device_constants_ensure(X->device));
     CU(cudaDeviceGetAttribute(&X->nsm, cudaDevAttrMultiProcessorCount, X->device));
@@ -755,7 +785,7 @@ static int ctx_create(Ctx **out, gpu_ulong p)
     if (!rc) rc = configure_kernels();
     if (!rc) rc = ctx_build_tables(X);
     if (!rc) {
-        cudaError_t e1 = cudaMalloc(&X->d_scale, sizeof(uint32_t) * (MAX_NP + 2) * (LOG_MAXM + 1) * MAX_NP);
+        cudaError_t e1 = cudaMalloc(&X->d_scale, sizeof(uint32_t) * (MAX_NP + 1 + NP3) * (LOG_MAXM + 1) * MAX_NP);
         cudaError_t e2 = cudaMalloc(&X->d_err, sizeof(int));
         cudaError_t e3 = cudaMalloc(&X->d_ticket, sizeof(unsigned long long));
         cudaError_t e4 = cudaHostAlloc(&X->h_err, sizeof(int), cudaHostAllocDefault);
@@ -950,24 +980,24 @@ static int plan_mpn(uint64_t an, uint64_t bn, MulPlan *P)
 }
 
 // pointwise scale: M^-1 (P/p_j)^-1 2^128, see k_rows / limb_redc
-static void fill_scale(const Ctx *X, int np, int logM, uint32_t *scale, int extra_redc)
+static void fill_scale(const HostTables &H, int np, int logM, uint32_t *scale, int extra_redc)
 {
     for (int j = 0; j < np; j++) {
         const uint32_t p = PRIMES[j];
         uint32_t s = h_invmod(h_powmod(2, logM, p), p);
-        s = h_mulmod(s, h_invmod(X->cof_red[np][j], p), p);
+        s = h_mulmod(s, h_invmod(H.cof_red[np][j], p), p);
         s = h_mulmod(s, h_powmod(2, 32 * (uint64_t)extra_redc, p), p);
         scale[j] = s;
     }
 }
 
 // pointwise scale of a 3 2^k-point transform: (3 2^k)^-1 (P/p_j)^-1 2^128
-static void fill_scale3(const Ctx *X, int np, int k, uint32_t *scale)
+static void fill_scale3(const HostTables &H, int np, int k, uint32_t *scale)
 {
     for (int j = 0; j < np; j++) {
         const uint32_t p = PRIMES[j];
         uint32_t s = h_invmod(h_mulmod(3, h_powmod(2, k, p), p), p);
-        s = h_mulmod(s, h_invmod(X->cof_red[np][j], p), p);
+        s = h_mulmod(s, h_invmod(H.cof_red[np][j], p), p);
         s = h_mulmod(s, h_powmod(2, 128, p), p);
         scale[j] = s;
     }
@@ -989,22 +1019,28 @@ static const uint32_t *scale_ptr(const Ctx *X, int np, int logM)
 {
     return X->d_scale + ((size_t)np * (LOG_MAXM + 1) + logM) * MAX_NP;
 }
-// scales of the 3 2^k-point transforms (NP3 primes), after the 2^logM ones
-static const uint32_t *scale3_ptr(const Ctx *X, int k)
+// scales of the 3 2^k-point transforms (1 .. NP3 primes), after the 2^logM ones
+static const uint32_t *scale3_ptr(const Ctx *X, int np, int k)
 {
-    return X->d_scale + ((size_t)(MAX_NP + 1) * (LOG_MAXM + 1) + k) * MAX_NP;
+    return X->d_scale + ((size_t)(MAX_NP + np) * (LOG_MAXM + 1) + k) * MAX_NP;
 }
 
-// pointwise scales for every (np, logM), uploaded once per context
-static int upload_scales(Ctx *X)
+// pointwise scales for every (np, logM)
+static void fill_scales(HostTables &H)
 {
-    std::vector<uint32_t> tab((size_t)(MAX_NP + 2) * (LOG_MAXM + 1) * MAX_NP, 0);
+    H.scales.assign((size_t)(MAX_NP + 1 + NP3) * (LOG_MAXM + 1) * MAX_NP, 0);
     for (int np = 1; np <= MAX_NP; np++)
         for (int lm = 0; lm <= LOG_MAXM; lm++)
-            fill_scale(X, np, lm, &tab[((size_t)np * (LOG_MAXM + 1) + lm) * MAX_NP], 4);
-    for (int k = 0; k <= LOG_MAXM; k++)
-        fill_scale3(X, NP3, k, &tab[((size_t)(MAX_NP + 1) * (LOG_MAXM + 1) + k) * MAX_NP]);
-    CU(cudaMemcpy(X->d_scale, tab.data(), tab.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+            fill_scale(H, np, lm, &H.scales[((size_t)np * (LOG_MAXM + 1) + lm) * MAX_NP], 4);
+    for (int np = 1; np <= NP3; np++)
+        for (int k = 0; k <= LOG_MAXM; k++)
+            fill_scale3(H, np, k, &H.scales[((size_t)(MAX_NP + np) * (LOG_MAXM + 1) + k) * MAX_NP]);
+}
+
+static int upload_scales(Ctx *X)
+{
+    const std::vector<uint32_t> &t = host_tables().scales;
+    CU(cudaMemcpy(X->d_scale, t.data(), t.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     return 0;
 }
 
@@ -1191,16 +1227,16 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
 // of 2^logMs words (logMs = k + 2).  The pointwise scale is folded into b's
 // twist as in launch_transforms (squarings keep it in the row pass).  With fz
 // the operands are integer polynomials (an, bn coefficients).
-static void launch_transforms3(const Ctx *X, int k, int logMs, const uint64_t *a, uint64_t an,
+static void launch_transforms3(const Ctx *X, int np, int k, int logMs, const uint64_t *a, uint64_t an,
                                const uint64_t *b, uint64_t bn, uint32_t *ra, uint32_t *rb, bool sq,
                                cudaStream_t st, TimingRecord *tr, cudaEvent_t b_ready,
                                const FzShape *fz = nullptr)
 {
-    const int np = NP3, r = k - LOGC3;
+    const int r = k - LOGC3;
     const int G = cols_per_tile3(r);
     const int C = 1 << LOGC3, rows = 3 << r;
     const size_t smem = (size_t)(padw(3 * (1 << r) * G) + 32) * sizeof(uint32_t);
-    const uint32_t *sc = scale3_ptr(X, k);
+    const uint32_t *sc = scale3_ptr(X, np, k);
     if (b_ready) cudaStreamWaitEvent(st, b_ready, 0);
     launch_dep((fz ? FWD_COLS3_FZ : FWD_COLS3)[r - LOG3_RMIN], dim3(np, C / G, sq ? 1 : 2), 512, smem, st, !b_ready,
                X->T, a, an, b, bn, ra, rb, logMs, k, sc, sq ? 0 : 2, fz ? *fz : FzShape{1, 1, 1});
@@ -1213,13 +1249,13 @@ static void launch_transforms3(const Ctx *X, int k, int logMs, const uint64_t *a
     timing_mark(tr, 3, st);
 }
 
-// The 3 2^k-point length for a whole product of L coefficients on the
-// default plan (np primes, 2^logM points), or 0 where the power of two stays
-// (beyond 3 2^(logM - 2), other prime counts, sizes outside the kernels').
+// The 3 2^k-point length for a product of L coefficients (np primes, 2^logM
+// points), or 0 where the power of two stays (beyond 3 2^(logM - 2), more primes
+// than have roots of that order, sizes outside the kernels').
 static int three_length(uint64_t L, int np, int logM)
 {
     const int k = logM - 2;
-    if (np != NP3 || k - LOGC3 < LOG3_RMIN || k - LOGC3 > LOG3_RMAX) return 0;
+    if (np > NP3 || k - LOGC3 < LOG3_RMIN || k - LOGC3 > LOG3_RMAX) return 0;
     return L <= (3ull << k) ? k : 0;
 }
 
@@ -1461,7 +1497,7 @@ static int mpn_mul_enqueue(Ctx *X, uint64_t *z, const uint64_t *a, uint64_t an,
         timing_mark(tr, 2, st);
         timing_mark(tr, 3, st);
     } else if (k3) {
-        launch_transforms3(X, k3, logM, a, an, b, bn, ra, rb, sq, st, tr, b_ready);
+        launch_transforms3(X, np, k3, logM, a, an, b, bn, ra, rb, sq, st, tr, b_ready);
     } else {
         // the product's residues: ra, or rb when b arrived late (launch_transforms)
         ra = launch_transforms(X, P.L, np, a, an, b, bn, ra, rb, sq, scale_ptr(X, np, logM), st, tr, nullptr, 1,
