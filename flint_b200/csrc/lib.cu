@@ -513,14 +513,14 @@ static const fwd_cols_fn FWD_COLS_FZ_C13[3] = {k_fwd_cols<9, tmpl_cols<9>(), tru
 static const inv_cols_fn INV_COLS_C13[3] = {k_inv_cols<9, tmpl_cols<9>(), 13>,
                                             k_inv_cols<10, tmpl_cols<10>(), 13>,
                                             k_inv_cols<11, tmpl_cols<11>(), 13>};
-// narrow tiles (a quarter of the columns, 128 threads) for columns of 2^5 to
-// 2^8 points (index logR - 5): small transforms get four times the CTAs
-static const fwd_cols_fn FWD_COLS_S[4] = {k_fwd_cols<5, cols_per_tile(5) / 4, false>,
-                                          k_fwd_cols<6, cols_per_tile(6) / 4, false>,
-                                          k_fwd_cols<7, cols_per_tile(7) / 4, false>,
-                                          k_fwd_cols<8, cols_per_tile(8) / 4, false>};
-static const inv_cols_fn INV_COLS_S[4] = {k_inv_cols<5, cols_per_tile(5) / 4>, k_inv_cols<6, cols_per_tile(6) / 4>,
-                                          k_inv_cols<7, cols_per_tile(7) / 4>, k_inv_cols<8, cols_per_tile(8) / 4>};
+// narrow tiles (half of the columns, 128 threads) for columns of 2^5 to 2^8
+// points (index logR - 5): small transforms get twice the CTAs
+static const fwd_cols_fn FWD_COLS_S[4] = {k_fwd_cols<5, cols_per_tile(5) / 2, false>,
+                                          k_fwd_cols<6, cols_per_tile(6) / 2, false>,
+                                          k_fwd_cols<7, cols_per_tile(7) / 2, false>,
+                                          k_fwd_cols<8, cols_per_tile(8) / 2, false>};
+static const inv_cols_fn INV_COLS_S[4] = {k_inv_cols<5, cols_per_tile(5) / 2>, k_inv_cols<6, cols_per_tile(6) / 2>,
+                                          k_inv_cols<7, cols_per_tile(7) / 2>, k_inv_cols<8, cols_per_tile(8) / 2>};
 static const fwd_cols_fn FWD_COLS_C14 = k_fwd_cols<11, tmpl_cols<11>(), false, 14>;
 static const fwd_cols_fn FWD_COLS_FZ_C14 = k_fwd_cols<11, tmpl_cols<11>(), true, 14>;
 static const inv_cols_fn INV_COLS_C14 = k_inv_cols<11, tmpl_cols<11>(), 14>;
@@ -650,8 +650,8 @@ static int batch_logC(int logM)
     return logM == 19 ? 11 : single_logC(logM);
 }
 // Shortest row for a transform of 2^logM points: columns at most 2^11 long,
-// and with 32 or more columns (the column kernel's 2^14-word tiles of
-// 2^(14 - logR) columns) rows at least one tile wide, which below 2^14
+// and with 32 or more columns (the column kernel's tiles are up to
+// 2^(14 - logR) columns wide) rows at least one tile wide, which below 2^14
 // points means at most 16 columns.
 static int min_logC(int logM)
 {
@@ -1111,9 +1111,9 @@ static LaunchShape row_launch_shape(const Ctx *X, const LaunchShape &L, int np, 
     return Lr;
 }
 
-// A column launch: the shape's 2^14-word tiles, or narrow ones (a quarter of
-// the columns) where the launch would have fewer than two CTAs per SM --
-// small transforms, whose column passes are bound by latency, not by HBM.
+// A column launch: the shape's 2^13-word tiles, or narrow ones (half of the
+// columns) where the launch would have fewer than four CTAs per SM -- small
+// transforms, whose column passes are bound by latency, not by HBM.
 struct ColLaunch {
     int G, grid, threads;
     size_t smem;
@@ -1124,10 +1124,10 @@ static ColLaunch col_launch(const Ctx *X, const LaunchShape &L, int np, int zdim
     const MulShape &S = L.S;
     ColLaunch c{S.G, L.col_grid, L.col_threads, L.col_smem, false};
     const int64_t want = 2 * (int64_t)X->nsm;
-    if (!fz && S.logR >= 5 && S.logR <= 8 && (int64_t)L.col_grid * np * zdim < want) {
-        c.G = S.G / 4;
-        c.grid = L.col_grid * 4;
-        c.threads = L.col_threads / 4;
+    if (!fz && S.logR >= 5 && S.logR <= 8 && (int64_t)L.col_grid * np * zdim < 2 * want) {
+        c.G = S.G / 2;
+        c.grid = L.col_grid * 2;
+        c.threads = L.col_threads / 2;
         c.smem = (size_t)(padw((1 << S.logR) * c.G) + 32) * sizeof(uint32_t);
         c.narrow = true;
     } else if (S.logR < 5) {
@@ -1238,14 +1238,14 @@ static void launch_transforms3(const Ctx *X, int np, int k, int logMs, const uin
     const size_t smem = (size_t)(padw(3 * (1 << r) * G) + 32) * sizeof(uint32_t);
     const uint32_t *sc = scale3_ptr(X, np, k);
     if (b_ready) cudaStreamWaitEvent(st, b_ready, 0);
-    launch_dep((fz ? FWD_COLS3_FZ : FWD_COLS3)[r - LOG3_RMIN], dim3(np, C / G, sq ? 1 : 2), 512, smem, st, !b_ready,
+    launch_dep((fz ? FWD_COLS3_FZ : FWD_COLS3)[r - LOG3_RMIN], dim3(np, C / G, sq ? 1 : 2), THREADS3, smem, st, !b_ready,
                X->T, a, an, b, bn, ra, rb, logMs, k, sc, sq ? 0 : 2, fz ? *fz : FzShape{1, 1, 1});
     timing_mark(tr, 1, st);
     const LaunchShape L = make_shape(logMs, LOGC3);   // row launch shape (one 2^13-point row per item)
     launch_rows(X, L, 5, ra, rb, logMs - LOGC3, np, sq ? sc : nullptr, sq ? 1 : 0, nullptr, 1, rows, st,
                 rows_dependent((size_t)3 << k, LOGC3));
     timing_mark(tr, 2, st);
-    launch_dep(INV_COLS3[r - LOG3_RMIN], dim3(C / G, np), 512, smem, st, true, X->T, ra, logMs, k);
+    launch_dep(INV_COLS3[r - LOG3_RMIN], dim3(C / G, np), THREADS3, smem, st, true, X->T, ra, logMs, k);
     timing_mark(tr, 3, st);
 }
 

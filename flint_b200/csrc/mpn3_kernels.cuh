@@ -35,8 +35,17 @@
 
 namespace fb {
 
-// columns per tile: 3 2^r rows x G columns of at most 3 2^13 words, G >= 8
-__host__ __device__ constexpr int cols_per_tile3(int logR) { return logR >= 10 ? 8 : (1 << (13 - logR)); }
+// columns per tile: 3 2^r rows x G columns of at most 3 2^12 words, G >= 8
+__host__ __device__ constexpr int cols_per_tile3(int logR) { return logR >= 9 ? 8 : (1 << (12 - logR)); }
+// threads per CTA: a tile of 3 2^12 words has 3 2^7 register sub-transforms of
+// 32, so every pass is a whole number of rounds, and three CTAs share an SM (56
+// registers).  Against tiles of 3 2^13 words, 512 threads and passes over one
+// third at a time: columns of 3 2^6 points (700000^2 limbs) forward 69.7 -> 60.7 us,
+// inverse 41.9 -> 32.4; 3 2^7 118.9 -> 115.3, 66.2 -> 51.8; 3 2^8 236 -> 222, 125
+// -> 99; 3 2^9 478 -> 485, 266 -> 201.  Two CTAs of up to 80 registers: 67.0 and
+// 36.1 at 3 2^6.
+constexpr int THREADS3 = 384;
+constexpr int CTAS3 = 3;
 
 __device__ __forceinline__ uint32_t table_power3(uint32_t e, const uint2* __restrict__ th3,
                                                  const uint2* __restrict__ tl3, uint32_t p)
@@ -74,16 +83,28 @@ __device__ __forceinline__ void twist32_3(uint32_t (&x)[32], uint32_t col, int s
 }
 
 // The strided passes of the three thirds of a column tile (three independent
-// transforms of 2^LOGL points down G columns, `third` words apart): each pass
-// runs on all three before one barrier, instead of three pass sequences with
-// a barrier after every pass.
+// transforms of 2^LOGL points down G columns, `third` words apart), each pass
+// over all of them before one barrier.
 template <int LOGL, int G, int QMAX, int H, int REM>
 __device__ __forceinline__ void gs_passes3(uint32_t* sm, int third, const uint2* __restrict__ tw, uint32_t p)
 {
     if constexpr (REM > 0) {
         constexpr int Q = balanced_pass<REM, QMAX>();
+        constexpr int E = 1 << Q, S = H >> (Q - 1), TOT = G * ((1 << LOGL) / E), SG = S * G;
+        static_assert(SG % 32 == 0, "unsupported pass stride");
 #pragma unroll 1
-        for (int t = 0; t < 3; t++) gs_pass_smem<LOGL, Q, H, G>(sm + t * third, 1, tw, p);
+        for (int f = threadIdx.x; f < 3 * TOT; f += THREADS3) {
+            const int t = f / TOT, v = f & (G - 1), s = (f - t * TOT) / G;
+            const int jj0 = s & (S - 1);
+            const int base = (s / S) * (2 * H) + jj0;
+            uint32_t* d = sm + t * third + padw(base * G) + v;
+            uint32_t x[E];
+#pragma unroll
+            for (int m = 0; m < E; m++) x[m] = d[padw(m * SG)];
+            gs_strided<Q, H, COL_FMA_ADDS>(x, tw, jj0, p);
+#pragma unroll
+            for (int m = 0; m < E; m++) d[padw(m * SG)] = x[m];
+        }
         __syncthreads();
         gs_passes3<LOGL, G, QMAX, (H >> Q), REM - Q>(sm, third, tw, p);
     }
@@ -93,8 +114,21 @@ __device__ __forceinline__ void ct_passes3(uint32_t* sm, int third, const uint2*
 {
     if constexpr (REM > 0) {
         constexpr int Q = balanced_pass<REM, QMAX>();
+        constexpr int E = 1 << Q, S = H, TOT = G * ((1 << LOGL) / E), SG = S * G;
+        static_assert(SG % 32 == 0, "unsupported pass stride");
 #pragma unroll 1
-        for (int t = 0; t < 3; t++) ct_pass_smem<LOGL, Q, H, G>(sm + t * third, 1, twi, p);
+        for (int f = threadIdx.x; f < 3 * TOT; f += THREADS3) {
+            const int t = f / TOT, v = f & (G - 1), s = (f - t * TOT) / G;
+            const int jj0 = s & (S - 1);
+            const int base = (s / S) * (S * E) + jj0;
+            uint32_t* d = sm + t * third + padw(base * G) + v;
+            uint32_t x[E];
+#pragma unroll
+            for (int m = 0; m < E; m++) x[m] = d[padw(m * SG)];
+            ct_strided<Q, H, COL_CT_FMA_ADDS>(x, twi, jj0, p);
+#pragma unroll
+            for (int m = 0; m < E; m++) d[padw(m * SG)] = x[m];
+        }
         __syncthreads();
         ct_passes3<LOGL, G, QMAX, (H << Q), REM - Q>(sm, third, twi, p);
     }
@@ -114,13 +148,13 @@ __device__ __forceinline__ void ct_strided_all3(uint32_t* sm, int third, const u
 
 // Forward column pass of a 3 2^k-point transform: limbs -> residues, radix-3
 // stage, three length-2^LOGR transforms, twist.  grid = (np, C / G, operands);
-// block 512; smem = padw(3 2^LOGR G) + 32 words.  logMs: log2 of the residue
+// block THREADS3; smem = padw(3 2^LOGR G) + 32 words.  logMs: log2 of the residue
 // plane stride; rows of C = 2^LOGC3 points.  fscale / fmask as in k_fwd_cols;
 // FZ: integer-polynomial operands (an, bn coefficients, chunk layout fz) as in
 // k_fwd_cols.
 constexpr int LOGC3 = 13;
 template <int LOGR, int G, bool FZ = false>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(THREADS3, CTAS3)
 k_fwd_cols3(DevTables T, const uint64_t* __restrict__ a, uint64_t an, const uint64_t* __restrict__ b,
             uint64_t bn, uint32_t* __restrict__ ra, uint32_t* __restrict__ rb, int logMs, int k,
             const uint32_t* __restrict__ fscale, int fmask, FzShape fz)
@@ -139,27 +173,27 @@ k_fwd_cols3(DevTables T, const uint64_t* __restrict__ a, uint64_t an, const uint
     pdl_wait();
 
     // limbs of rows 0 .. 3R' - 1 (element n = u C + i; zero beyond the operand).
-    // blockDim == 512: thread t loads rows u_t + k 512/G of its column, so its
-    // shared offsets are compile-time constants and its global address a
-    // pointer bump; the in-range loads are counted once (a shift)
+    // thread t loads rows u_t + k THREADS3/G of its column, so its shared offsets
+    // are compile-time constants and its global address a pointer bump; the
+    // in-range loads are counted once
     {
-        constexpr int K = 3 * RP * G / 512;
-        constexpr int ROWS_PER = 512 / G;
+        constexpr int K = 3 * RP * G / THREADS3;
+        constexpr int ROWS_PER = THREADS3 / G;
         const int t = threadIdx.x;
         const int u_t = t / G, c = t & (G - 1);
         const uint64_t n0 = (uint64_t)u_t * C + i0 + c;
-        static_assert(RP * G == 8192, "tiles of 3 2^13 words");
+        static_assert(3 * RP * G % THREADS3 == 0 && THREADS3 % G == 0 && THREADS3 % 32 == 0, "whole rounds");
         uint32_t* d = sm + padw(u_t * G) + c;
         if constexpr (!FZ) {
-            constexpr int lstep = LOGR - 4 + LOGC3;   // log2(ROWS_PER C): ROWS_PER = 2^(LOGR - 4)
+            constexpr uint64_t step = (uint64_t)ROWS_PER * C;
             int kin = 0;
             if (n0 < xn) {
-                const uint64_t q = ((xn - n0 - 1) >> lstep) + 1;
+                const uint64_t q = (xn - n0 - 1) / step + 1;
                 kin = q < (uint64_t)K ? (int)q : K;
             }
             const uint64_t* px = x + n0;
 #pragma unroll 8
-            for (int k = 0; k < K; k++, px += (size_t)ROWS_PER * C)
+            for (int k = 0; k < K; k++, px += step)
                 d[k * (ROWS_PER * G + ROWS_PER * G / 32)] = k < kin ? limb_redc(*px, p, P.pneg_inv, P.c32) : 0u;
         } else {
             // chunk (n mod S) of coefficient n / S, with the slot, the chunk
@@ -236,9 +270,9 @@ k_fwd_cols3(DevTables T, const uint64_t* __restrict__ a, uint64_t an, const uint
 
 // Inverse column pass of a 3 2^k-point transform, in place: untwist, three
 // length-2^LOGR inverse transforms, inverse radix-3 stage.
-// grid = (C / G, np); block 512; smem as k_fwd_cols3.
+// grid = (C / G, np); block THREADS3; smem as k_fwd_cols3.
 template <int LOGR, int G>
-__global__ void __launch_bounds__(512)
+__global__ void __launch_bounds__(THREADS3, CTAS3)
 k_inv_cols3(DevTables T, uint32_t* __restrict__ ra, int logMs, int k)
 {
     extern __shared__ uint32_t sm[];

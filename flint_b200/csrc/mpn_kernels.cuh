@@ -94,11 +94,15 @@ struct MulShape {
     int G;                 // columns per column-pass tile
 };
 
-// columns per tile for a column length 2^logR: 64 KB tiles, at least 8
-// columns (32-byte row segments)
+// columns per tile for a column length 2^logR: 32 KB tiles (256 threads, four
+// CTAs per SM whose loads, levels and stores overlap), at least 8 columns
+// (32-byte row segments).  Against 64 KB tiles of 512 threads, two per SM, which
+// 2^11-point columns keep: columns of 2^8 points (2^20 x 2^20 limbs) forward 74.2 ->
+// 68.3 us, inverse 36.6 -> 32.0; 2^9 137.7 -> 125.7, 61.6 -> 57.3; 2^10 284.0 ->
+// 282.2, 135.0 -> 128.8.
 __host__ __device__ constexpr int cols_per_tile(int logR)
 {
-    return logR >= 11 ? 8 : (1 << (14 - logR));
+    return logR >= 10 ? 8 : (1 << (13 - logR));
 }
 
 // w^e for e in units of the largest transform, from the two-level tables
@@ -252,7 +256,7 @@ fwd_cols_body(DevTables T, const uint64_t* __restrict__ a, uint64_t an,
     const uint64_t M = (uint64_t)1 << logM;
     const int tot = R * GR;
     // threads of a tile with columns of 2^5 points or more: one per 32-point
-    // column segment (512 for the 2^14-word tiles, fewer for narrow ones)
+    // column segment (256 for the 2^13-word tiles, 512 for 2^14, fewer for narrow ones)
     constexpr int NT = G ? (G * R / 32 < 512 ? G * R / 32 : 512) : 512;
     constexpr int PNT = NT + NT / 32;     // padw(NT)
 

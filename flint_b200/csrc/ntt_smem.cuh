@@ -47,10 +47,10 @@ constexpr int MAX_NP = 7;
 #ifndef FB_COL_FMA_ADDS
 #define FB_COL_FMA_ADDS 0
 #endif
-// inverse column passes: fused reductions with FMA-pipe twiddle-1 butterflies
-// (F = -2: 0.561 -> 0.539 ms against F = 0)
+// inverse column passes: fused reductions, twiddle-1 butterflies on the ALU
+// (2^25 points: F = 0 0.565 ms, F = -2 0.530, F = -1 0.517)
 #ifndef FB_COL_CT_FMA_ADDS
-#define FB_COL_CT_FMA_ADDS (-2)
+#define FB_COL_CT_FMA_ADDS (-1)
 #endif
 #ifndef FB_ROW_GS_FMA_ADDS
 #define FB_ROW_GS_FMA_ADDS (-1)
