@@ -781,6 +781,12 @@ inv_cols_body(DevTables T, uint32_t* __restrict__ ra, int logC, int gcols,
     const uint32_t mmask = (uint32_t)(((uint64_t)1 << logM) - 1);
 
     if constexpr (LOGR >= 5) {
+        // element u of column v of a split product's chunk
+        auto chunk_store = [&](int u, int v, uint32_t x) {
+            uint32_t* __restrict__ out = co.acc + ((size_t)j << co.logMf) + co.shift;
+            const uint64_t n = (uint64_t)u * C + i0 + v;
+            if (n < co.nvalid) out[n] = n < co.overlap ? add_mod(out[n], x, p) : x;
+        };
         constexpr int NS = R / 32;
         for (int f = threadIdx.x; f < G * NS; f += blockDim.x) {
             const int v = f & (G - 1), s = f / G;
@@ -791,34 +797,35 @@ inv_cols_body(DevTables T, uint32_t* __restrict__ ra, int logC, int gcols,
             for (int m = 0; m < 32; m++) xr[m] = src[(size_t)m * C];
             twist32<LOGR>(xr, col, s, logM, th, tl, P);
             ct_contig<5, COL_CT_FMA_ADDS>(xr, c_w32[j], p);
-            const int pb = 33 * G * s + v;
+            if constexpr (LOGR == 5) {
+                // the whole column is in registers
+                if (!co.acc) {
+                    uint32_t* dst = buf + col;
 #pragma unroll
-            for (int m = 0; m < 32; m++) sm[pb + padw(m * G)] = xr[m];
-        }
-        __syncthreads();
-        ct_strided_all<LOGR, G>(sm, 1, T.twi + (size_t)j * TW_SZ, p);
-        // blockDim == G R / 32 == NT: thread t stores rows u_t + k NT/G of
-        // its column (the inverse of the forward pass's load mapping)
-        constexpr int NT = G * R / 32 < 512 ? G * R / 32 : 512;
-        constexpr int PNT = NT + NT / 32;     // padw(NT)
-        const int t = threadIdx.x;
-        const int u_t = t / G, c = t & (G - 1);
-        const size_t step = (size_t)(NT / G) * C;
-        const uint32_t* s_ = sm + padw(u_t * G) + c;
-        if (!co.acc) {
-            uint32_t* dst = buf + (size_t)u_t * C + i0 + c;
-#pragma unroll 8
-            for (int k = 0; k < R * G / NT; k++) dst[k * step] = s_[k * PNT];
-        } else {
-            uint32_t* __restrict__ out = co.acc + ((size_t)j << co.logMf) + co.shift;
-            const uint64_t n0 = (uint64_t)u_t * C + i0 + c;
-#pragma unroll 8
-            for (int k = 0; k < R * G / NT; k++) {
-                const uint64_t n = n0 + (uint64_t)k * step;
-                if (n < co.nvalid) {
-                    const uint32_t v = s_[k * PNT];
-                    out[n] = n < co.overlap ? add_mod(out[n], v, p) : v;
+                    for (int m = 0; m < 32; m++) dst[(size_t)m * C] = xr[m];
+                } else {
+#pragma unroll
+                    for (int m = 0; m < 32; m++) chunk_store(m, v, xr[m]);
                 }
+            } else {
+                const int pb = 33 * G * s + v;
+#pragma unroll
+                for (int m = 0; m < 32; m++) sm[pb + padw(m * G)] = xr[m];
+            }
+        }
+        if constexpr (LOGR > 5) {
+            __syncthreads();
+            // the last strided pass stores from registers: the tile's way back
+            // through shared memory and its barrier cost columns of 2^10 points
+            // 127.8 us against 120.8, of 2^9 57.4 against 53.7 (2^11: even)
+            const uint2* __restrict__ twi = T.twi + (size_t)j * TW_SZ;
+            if (!co.acc) {
+                uint32_t* dst = buf + i0;
+                ct_passes_cols_out<LOGR, G, 4, 32, LOGR - 5>(sm, twi, p, [&](int u, int v, uint32_t x) {
+                    dst[(size_t)u * C + v] = x;
+                });
+            } else {
+                ct_passes_cols_out<LOGR, G, 4, 32, LOGR - 5>(sm, twi, p, chunk_store);
             }
         }
     } else if constexpr (LOGR > 0) {

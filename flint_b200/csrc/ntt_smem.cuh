@@ -483,6 +483,35 @@ __device__ __forceinline__ void ct_passes_out(uint32_t* sm, const uint2* __restr
     }
 }
 
+// The column counterpart: the last inverse pass of a tile of G columns hands
+// element u of column v to store(u, v, value) from registers -- consecutive
+// threads take consecutive columns.
+template <int LOGL, int G, int QMAX, int H, int REM, class Store>
+__device__ __forceinline__ void ct_passes_cols_out(uint32_t* sm, const uint2* __restrict__ twi, uint32_t p,
+                                                   const Store& store)
+{
+    constexpr int Q = balanced_pass<REM, QMAX>();
+    if constexpr (REM > Q) {
+        ct_pass_smem<LOGL, Q, H, G>(sm, 1, twi, p);
+        __syncthreads();
+        ct_passes_cols_out<LOGL, G, QMAX, (H << Q), REM - Q>(sm, twi, p, store);
+    } else {
+        constexpr int E = 1 << Q, S = H, NSUB = (1 << LOGL) / E;
+        static_assert(S * G % 32 == 0 && NSUB == S, "the last pass spans the column");
+#pragma unroll PASS_UNROLL
+        for (int f = threadIdx.x; f < G * NSUB; f += blockDim.x) {
+            const int v = f & (G - 1), s = f / G;
+            const uint32_t* d = sm + padw(s * G) + v;
+            uint32_t x[E];
+#pragma unroll
+            for (int m = 0; m < E; m++) x[m] = d[padw(m * S * G)];
+            ct_strided<Q, H, COL_CT_FMA_ADDS>(x, twi, s, p);
+#pragma unroll
+            for (int m = 0; m < E; m++) store(s + m * S, v, x[m]);
+        }
+    }
+}
+
 // ct_strided_all for one row (rows layout, nv = 1) whose final pass stores
 // the row to global memory at `out`; needs LOGL > LOGE.  The shared buffer
 // is read, not written, by the final pass.
