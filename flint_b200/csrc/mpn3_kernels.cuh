@@ -172,76 +172,75 @@ k_fwd_cols3(DevTables T, const uint64_t* __restrict__ a, uint64_t an, const uint
     const uint32_t p = P.p;
     pdl_wait();
 
-    // limbs of rows 0 .. 3R' - 1 (element n = u C + i; zero beyond the operand).
-    // thread t loads rows u_t + k THREADS3/G of its column, so its shared offsets
-    // are compile-time constants and its global address a pointer bump; the
-    // in-range loads are counted once
-    {
-        constexpr int K = 3 * RP * G / THREADS3;
-        constexpr int ROWS_PER = THREADS3 / G;
-        const int t = threadIdx.x;
-        const int u_t = t / G, c = t & (G - 1);
-        const uint64_t n0 = (uint64_t)u_t * C + i0 + c;
-        static_assert(3 * RP * G % THREADS3 == 0 && THREADS3 % G == 0 && THREADS3 % 32 == 0, "whole rounds");
-        uint32_t* d = sm + padw(u_t * G) + c;
-        if constexpr (!FZ) {
-            constexpr uint64_t step = (uint64_t)ROWS_PER * C;
-            int kin = 0;
-            if (n0 < xn) {
-                const uint64_t q = (xn - n0 - 1) / step + 1;
-                kin = q < (uint64_t)K ? (int)q : K;
-            }
-            const uint64_t* px = x + n0;
-#pragma unroll 8
-            for (int k = 0; k < K; k++, px += step)
-                d[k * (ROWS_PER * G + ROWS_PER * G / 32)] = k < kin ? limb_redc(*px, p, P.pneg_inv, P.c32) : 0u;
-        } else {
-            // chunk (n mod S) of coefficient n / S, with the slot, the chunk
-            // and the limb offset advanced incrementally (as in k_fwd_cols)
-            const uint32_t S = fz.S, xw = opb ? fz.wb : fz.wa;
-            const uint32_t step = (uint32_t)ROWS_PER * C;
-            uint32_t ci = (uint32_t)n0 / S, ck = (uint32_t)n0 - ci * S;
-            const uint32_t sq = step / S, sr = step - sq * S;
-            size_t off = (size_t)ci * xw + ck;
-            const size_t doff = (size_t)sq * xw + sr;
-#pragma unroll 8
-            for (int k = 0; k < K; k++) {
-                uint32_t r = 0;
-                if (ck < xw && ci < xn) {
-                    const uint64_t v = x[off];
-                    r = limb_redc(v, p, P.pneg_inv, P.c32);
-                    // a negative top limb stands for v - 2^64
-                    if (ck == xw - 1 && (int64_t)v < 0) r = sub_mod(r, P.c32, p);
-                }
-                d[k * (ROWS_PER * G + ROWS_PER * G / 32)] = r;
-                ci += sq;
-                ck += sr;
-                off += doff;
-                if (ck >= S) {
-                    ck -= S;
-                    ci++;
-                    off -= (size_t)(S - xw);   // S >= xw
-                }
-            }
-        }
-    }
-    __syncthreads();
+    // limbs (element n = u C + i; zero beyond the operand) straight into the
     // radix-3 stage: (u1, u1 + R', u1 + 2R') -> t0, t1 omega^u1, t2 omega^(2 u1)
     {
         const uint2 cw = T.w3c[(size_t)j * 2];
         const uint2* __restrict__ tw3 = T.tw3f + (size_t)j * TW3_SZ;
-        for (int f = threadIdx.x; f < RP * G; f += blockDim.x) {
-            const int u1 = f / G, c = f & (G - 1);
-            const int o0 = padw(u1 * G) + c, o1 = padw((u1 + RP) * G) + c, o2 = padw((u1 + 2 * RP) * G) + c;
-            const uint32_t x0 = sm[o0], x1 = sm[o1], x2 = sm[o2];
+        auto stage = [&](int u1, int c, uint32_t x0, uint32_t x1, uint32_t x2) {
             const uint32_t s = add_mod(x1, x2, p), d = sub_mod(x1, x2, p);
             const uint32_t cd = mul_shoup(d, cw.x, cw.y, p);
             const uint32_t h = sub_mod(add_mod(x0, x0, p), s, p);  // 2 x0 - a
             const int e = u1 << (LOG_R3 - LOGR);
             const uint2 w1 = tw3[e], w2 = tw3[2 * e];
-            sm[o0] = add_mod(x0, s, p);
-            sm[o1] = mul_shoup(h + cd, w1.x, w1.y, p);             // h + cd < 2p: any 32-bit input
-            sm[o2] = mul_shoup(h - cd + p, w2.x, w2.y, p);
+            uint32_t* o = sm + padw(u1 * G) + c;
+            o[0] = add_mod(x0, s, p);
+            o[padw(RP * G)] = mul_shoup(h + cd, w1.x, w1.y, p);    // h + cd < 2p: any 32-bit input
+            o[2 * padw(RP * G)] = mul_shoup(h - cd + p, w2.x, w2.y, p);
+        };
+        constexpr uint32_t third = (uint32_t)RP * C;             // elements between a triple's rows
+        if constexpr (!FZ) {
+#pragma unroll 2
+            for (int f = threadIdx.x; f < RP * G; f += THREADS3) {
+                const int u1 = f / G, c = f & (G - 1);
+                const uint64_t n = (uint64_t)u1 * C + i0 + c;
+                const uint64_t v0 = n < xn ? x[n] : 0ull, v1 = n + third < xn ? x[n + third] : 0ull,
+                               v2 = n + 2 * (uint64_t)third < xn ? x[n + 2 * (uint64_t)third] : 0ull;
+                stage(u1, c, limb_redc(v0, p, P.pneg_inv, P.c32), limb_redc(v1, p, P.pneg_inv, P.c32),
+                      limb_redc(v2, p, P.pneg_inv, P.c32));
+            }
+        } else {
+            // chunk (n mod S) of coefficient n / S: the slot, the chunk and the
+            // limb offset advance by fixed amounts, from row to row of a triple
+            // and from triple to triple (as in k_fwd_cols)
+            const uint32_t S = fz.S, xw = opb ? fz.wb : fz.wa;
+            const uint32_t step = (uint32_t)(THREADS3 / G) * C;
+            const uint32_t sq = step / S, sr = step - sq * S, tq = third / S, tr = third - tq * S;
+            const size_t doff = (size_t)sq * xw + sr, toff = (size_t)tq * xw + tr;
+            const uint32_t n0 = (uint32_t)(threadIdx.x / G) * C + i0 + (threadIdx.x & (G - 1));
+            uint32_t ci = n0 / S, ck = n0 - ci * S;
+            size_t off = (size_t)ci * xw + ck;
+            auto advance = [&](uint32_t& i, uint32_t& k, size_t& o, uint32_t q, uint32_t r, size_t d) {
+                i += q;
+                k += r;
+                o += d;
+                if (k >= S) {
+                    k -= S;
+                    i++;
+                    o -= (size_t)(S - xw);   // S >= xw: one slot on, minus the chunks it carries
+                }
+            };
+            auto value = [&](uint32_t i, uint32_t k, size_t o) {
+                uint32_t r = 0;
+                if (k < xw && i < xn) {
+                    const uint64_t v = x[o];
+                    r = limb_redc(v, p, P.pneg_inv, P.c32);
+                    // a negative top limb stands for v - 2^64
+                    if (k == xw - 1 && (int64_t)v < 0) r = sub_mod(r, P.c32, p);
+                }
+                return r;
+            };
+            for (int f = threadIdx.x; f < RP * G; f += THREADS3) {
+                uint32_t i = ci, k = ck, y[3];
+                size_t o = off;
+#pragma unroll
+                for (int t = 0; t < 3; t++) {
+                    y[t] = value(i, k, o);
+                    if (t < 2) advance(i, k, o, tq, tr, toff);
+                }
+                stage(f / G, f & (G - 1), y[0], y[1], y[2]);
+                advance(ci, ck, off, sq, sr, doff);
+            }
         }
     }
     __syncthreads();

@@ -260,7 +260,45 @@ fwd_cols_body(DevTables T, const uint64_t* __restrict__ a, uint64_t an,
     constexpr int NT = G ? (G * R / 32 < 512 ? G * R / 32 : 512) : 512;
     constexpr int PNT = NT + NT / 32;     // padw(NT)
 
-    if (LOGR >= 5 && (FZ || xn <= M)) {
+    // Columns over 2^13-point rows run their first strided pass straight from the
+    // limbs, without the tile's round trip through shared memory and one barrier:
+    // 2^9-point columns 125.6 -> 121.1 us, 2^10 282.4 -> 268.6, 2^11 615 -> 578.
+    // 2^14-point rows lost (1130 -> 1170 us) and shorter ones gained nothing; the
+    // chunk loads of integer polynomials need a division per sub-transform.
+    constexpr bool FUSED = !FZ && LC == 13;
+    constexpr int Q1 = LOGR > 5 ? balanced_pass<(LOGR > 5 ? LOGR - 5 : 1), 4>() : 1;   // levels of the first strided pass
+    bool first_done = false;
+    if (FUSED && xn <= M) {
+        // the first strided pass straight from the limbs: sub-transform s of
+        // column v takes rows s + m S
+        if constexpr (FUSED) {
+            constexpr int E = 1 << Q1, S = R / E, GG = G ? G : 1;
+            const uint2* __restrict__ tw = T.twf + (size_t)j * TW_SZ;
+            constexpr int LS = LOGR - Q1;     // S = 2^LS rows
+#pragma unroll 1
+            for (int f = threadIdx.x; f < GG * S; f += NT) {
+                const int v = f & (GG - 1), s = f / GG;
+                const uint64_t n = ((uint64_t)s << logC) + i0 + v;
+                int kin = 0;
+                if (n < xn) {
+                    const uint64_t q = ((xn - n - 1) >> (LS + logC)) + 1;
+                    kin = q < (uint64_t)E ? (int)q : E;
+                }
+                const uint64_t* px = x + n;
+                uint64_t lim[E];
+#pragma unroll
+                for (int m = 0; m < E; m++) lim[m] = m < kin ? px[(size_t)m << (LS + logC)] : 0ull;
+                uint32_t xr[E];
+#pragma unroll
+                for (int m = 0; m < E; m++) xr[m] = limb_redc(lim[m], p, P.pneg_inv, P.c32);
+                gs_strided<Q1, R / 2, COL_FMA_ADDS>(xr, tw, s, p);
+                uint32_t* d = sm + padw(s * GG) + v;
+#pragma unroll
+                for (int m = 0; m < E; m++) d[padw(m * S * GG)] = xr[m];
+            }
+            first_done = true;
+        }
+    } else if (LOGR >= 5 && (FZ || xn <= M)) {
         // blockDim == G R / 32 == NT: thread t loads elements t + NT k, i.e.
         // rows u_t + k NT/G of its fixed column; shared offsets are constants
         const int t = threadIdx.x;
@@ -356,7 +394,15 @@ fwd_cols_body(DevTables T, const uint64_t* __restrict__ a, uint64_t an,
         // pointwise scale folded into this operand's twist (fmask bit 0: the
         // first operand, bit 1: the second)
         const uint32_t fsc = (fmask >> (opb ? 1 : 0)) & 1 ? fscale[j] : 0u;
-        gs_strided_all<LOGR, G>(sm, 1, T.twf + (size_t)j * TW_SZ, p);
+        if constexpr (FUSED) {
+            if (!first_done) {
+                gs_pass_smem<LOGR, Q1, R / 2, G>(sm, 1, T.twf + (size_t)j * TW_SZ, p);
+                __syncthreads();
+            }
+            gs_passes<LOGR, G, 4, ((R / 2) >> Q1), LOGR - 5 - Q1>(sm, 1, T.twf + (size_t)j * TW_SZ, p);
+        } else {
+            gs_strided_all<LOGR, G>(sm, 1, T.twf + (size_t)j * TW_SZ, p);
+        }
         constexpr int NS = R / 32;
         for (int f = threadIdx.x; f < G * NS; f += blockDim.x) {
             const int v = f & (G - 1), s = f / G;
