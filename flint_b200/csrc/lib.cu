@@ -486,7 +486,7 @@ static int ctx_build_tables(Ctx *X)
 typedef void (*fwd_cols_fn)(DevTables, const uint64_t *, uint64_t, const uint64_t *, uint64_t,
                             uint32_t *, uint32_t *, int, int, const InstDesc *, int, FzShape,
                             const uint32_t *, int);
-typedef void (*inv_cols_fn)(DevTables, uint32_t *, int, int, const InstDesc *, ChunkOut);
+typedef void (*inv_cols_fn)(DevTables, uint32_t *, int, int, const InstDesc *, ChunkOut, const uint32_t *);
 typedef void (*rows_fn)(DevTables, uint32_t *, const uint32_t *, int, int, int, const uint32_t *,
                         int, const InstDesc *, int, int);
 
@@ -521,14 +521,23 @@ static const fwd_cols_fn FWD_COLS_S[4] = {k_fwd_cols<5, cols_per_tile(5) / 2, fa
                                           k_fwd_cols<8, cols_per_tile(8) / 2, false>};
 static const inv_cols_fn INV_COLS_S[4] = {k_inv_cols<5, cols_per_tile(5) / 2>, k_inv_cols<6, cols_per_tile(6) / 2>,
                                           k_inv_cols<7, cols_per_tile(7) / 2>, k_inv_cols<8, cols_per_tile(8) / 2>};
+// the same for squarings (SC, columns of 2^5 points or more)
+#define FB_SC(r, ...) k_inv_cols<r, cols_per_tile(r) __VA_ARGS__, true>
+static const inv_cols_fn INV_COLS_SC[7] = {FB_SC(5, , 0), FB_SC(6, , 0), FB_SC(7, , 0), FB_SC(8, , 0),
+                                           FB_SC(9, , 0), FB_SC(10, , 0), FB_SC(11, , 0)};
+static const inv_cols_fn INV_COLS_SC_S[4] = {FB_SC(5, / 2, 0), FB_SC(6, / 2, 0), FB_SC(7, / 2, 0), FB_SC(8, / 2, 0)};
+static const inv_cols_fn INV_COLS_SC_C13[3] = {FB_SC(9, , 13), FB_SC(10, , 13), FB_SC(11, , 13)};
+static const inv_cols_fn INV_COLS_SC_C14 = FB_SC(11, , 14);
+#undef FB_SC
 static const fwd_cols_fn FWD_COLS_C14 = k_fwd_cols<11, tmpl_cols<11>(), false, 14>;
 static const fwd_cols_fn FWD_COLS_FZ_C14 = k_fwd_cols<11, tmpl_cols<11>(), true, 14>;
 static const inv_cols_fn INV_COLS_C14 = k_inv_cols<11, tmpl_cols<11>(), 14>;
 
-// columns of 3 2^r points, r = 5 .. 10 (index r - 5)
+// columns of 3 2^r points, r = 5 .. 10 (index r - 5; the inverse's second six for
+// squarings)
 typedef void (*fwd_cols3_fn)(DevTables, const uint64_t *, uint64_t, const uint64_t *, uint64_t, uint32_t *,
                              uint32_t *, int, int, const uint32_t *, int, FzShape);
-typedef void (*inv_cols3_fn)(DevTables, uint32_t *, int, int);
+typedef void (*inv_cols3_fn)(DevTables, uint32_t *, int, int, const uint32_t *);
 constexpr int LOG3_RMIN = 5, LOG3_RMAX = 10;
 static const fwd_cols3_fn FWD_COLS3[6] = {
     k_fwd_cols3<5, cols_per_tile3(5)>, k_fwd_cols3<6, cols_per_tile3(6)>, k_fwd_cols3<7, cols_per_tile3(7)>,
@@ -538,9 +547,12 @@ static const fwd_cols3_fn FWD_COLS3_FZ[6] = {
     k_fwd_cols3<5, cols_per_tile3(5), true>, k_fwd_cols3<6, cols_per_tile3(6), true>,
     k_fwd_cols3<7, cols_per_tile3(7), true>, k_fwd_cols3<8, cols_per_tile3(8), true>,
     k_fwd_cols3<9, cols_per_tile3(9), true>, k_fwd_cols3<10, cols_per_tile3(10), true>};
-static const inv_cols3_fn INV_COLS3[6] = {
+static const inv_cols3_fn INV_COLS3[12] = {
     k_inv_cols3<5, cols_per_tile3(5)>, k_inv_cols3<6, cols_per_tile3(6)>, k_inv_cols3<7, cols_per_tile3(7)>,
-    k_inv_cols3<8, cols_per_tile3(8)>, k_inv_cols3<9, cols_per_tile3(9)>, k_inv_cols3<10, cols_per_tile3(10)>};
+    k_inv_cols3<8, cols_per_tile3(8)>, k_inv_cols3<9, cols_per_tile3(9)>, k_inv_cols3<10, cols_per_tile3(10)>,
+    k_inv_cols3<5, cols_per_tile3(5), true>, k_inv_cols3<6, cols_per_tile3(6), true>,
+    k_inv_cols3<7, cols_per_tile3(7), true>, k_inv_cols3<8, cols_per_tile3(8), true>,
+    k_inv_cols3<9, cols_per_tile3(9), true>, k_inv_cols3<10, cols_per_tile3(10), true>};
 
 // the column kernels for a transform shape
 static fwd_cols_fn fwd_cols_kernel(int logR, int logC, bool fz = false)
@@ -549,8 +561,13 @@ static fwd_cols_fn fwd_cols_kernel(int logR, int logC, bool fz = false)
     if (logR >= 9 && logR <= 11 && logC == 13) return (fz ? FWD_COLS_FZ_C13 : FWD_COLS_C13)[logR - 9];
     return (fz ? FWD_COLS_FZ : FWD_COLS)[logR];
 }
-static inv_cols_fn inv_cols_kernel(int logR, int logC)
+static inv_cols_fn inv_cols_kernel(int logR, int logC, bool sc = false)
 {
+    if (sc) {
+        if (logR == 11 && logC == 14) return INV_COLS_SC_C14;
+        if (logR >= 9 && logR <= 11 && logC == 13) return INV_COLS_SC_C13[logR - 9];
+        return INV_COLS_SC[logR - 5];
+    }
     if (logR == 11 && logC == 14) return INV_COLS_C14;
     if (logR >= 9 && logR <= 11 && logC == 13) return INV_COLS_C13[logR - 9];
     return INV_COLS[logR];
@@ -751,7 +768,13 @@ static int configure_kernels()
     CU(cudaFuncSetAttribute(FWD_COLS_C14, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     CU(cudaFuncSetAttribute(FWD_COLS_FZ_C14, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     CU(cudaFuncSetAttribute(INV_COLS_C14, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+    for (int r = 0; r < 7; r++)
+        CU(cudaFuncSetAttribute(INV_COLS_SC[r], cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+    for (int r = 0; r < 3; r++)
+        CU(cudaFuncSetAttribute(INV_COLS_SC_C13[r], cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
+    CU(cudaFuncSetAttribute(INV_COLS_SC_C14, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
     for (int r = 0; r < 6; r++) {
+        CU(cudaFuncSetAttribute(INV_COLS3[r + 6], cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
         CU(cudaFuncSetAttribute(FWD_COLS3[r], cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
         CU(cudaFuncSetAttribute(FWD_COLS3_FZ[r], cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
         CU(cudaFuncSetAttribute(INV_COLS3[r], cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024));
@@ -1154,13 +1177,15 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
     const ColLaunch cf = col_launch(X, L, np, zdim, fz != nullptr);
     const ColLaunch ci = col_launch(X, L, np, ni, false);
     const fwd_cols_fn fwd = cf.narrow ? FWD_COLS_S[S.logR - 5] : fwd_cols_kernel(S.logR, S.logC, fz != nullptr);
-    const inv_cols_fn inv = ci.narrow ? INV_COLS_S[S.logR - 5] : inv_cols_kernel(S.logR, S.logC);
-    const FzShape shape = fz ? *fz : FzShape{1, 1, 1};
     // Products of two operands whose columns are long enough for the
     // per-thread twist (2^5 points or more) fold the pointwise scale into
     // b's twist factors, so the row pass multiplies the spectra once instead
-    // of twice; squarings keep the scale in the row pass.
-    const bool fold = !(sq && !desc) && S.logR >= 5;
+    // of twice; squarings fold it into the inverse column pass's untwist.
+    const bool square = sq && !desc;
+    const bool fold = !square && S.logR >= 5, fold_inv = square && S.logR >= 5;
+    const inv_cols_fn inv = ci.narrow ? (fold_inv ? INV_COLS_SC_S : INV_COLS_S)[S.logR - 5]
+                                      : inv_cols_kernel(S.logR, S.logC, fold_inv);
+    const FzShape shape = fz ? *fz : FzShape{1, 1, 1};
     // a batch's launches are the nodes of its graph, without launch gaps
     const bool dep = !desc;
     const int R = 1 << S.logR;
@@ -1200,7 +1225,7 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
             launch_rows(X, L, 5, rb, ra, S.logR, np, nullptr, 2, nullptr, 1, R, st, false);
             timing_mark(tr, 2, st);
             inv<<<dim3(ci.grid, np, 1), ci.threads, ci.smem, st>>>(X->T, rb, S.logC, ci.G, nullptr,
-                                                                   ChunkOut{nullptr, 0, 0, 0, 0});
+                                                                   ChunkOut{nullptr, 0, 0, 0, 0}, nullptr);
             timing_mark(tr, 3, st);
             return rb;
         }
@@ -1212,12 +1237,12 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
     timing_mark(tr, 1, st);
     const LaunchShape Lr = row_launch_shape(X, L, np, ni);
     const int loge = rows_loge(X, Lr, np, ni);
-    launch_rows(X, Lr, loge, ra, rb, S.logR, np, fold ? nullptr : d_scale, (sq && !desc) ? 1 : 0, desc, ni, R, st,
+    launch_rows(X, Lr, loge, ra, rb, S.logR, np, fold || fold_inv ? nullptr : d_scale, square ? 1 : 0, desc, ni, R, st,
                 dep && rows_dependent((size_t)1 << (S.logR + S.logC), S.logC, loge));
     timing_mark(tr, 2, st);
     if (S.logR > 0)
         launch_dep(inv, dim3(ci.grid, np, ni), ci.threads, ci.smem, st, dep && S.logR < 9, X->T, ra, S.logC, ci.G, desc,
-                   co ? *co : ChunkOut{nullptr, 0, 0, 0, 0});
+                   co ? *co : ChunkOut{nullptr, 0, 0, 0, 0}, fold_inv ? d_scale : nullptr);
     timing_mark(tr, 3, st);
     return ra;
 }
@@ -1225,7 +1250,7 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
 // Transform of M = 3 2^k points (k - 13 in [LOG3_RMIN, LOG3_RMAX]): columns of
 // 3 2^(k - 13) points with a radix-3 stage, 2^13-point rows; residue planes
 // of 2^logMs words (logMs = k + 2).  The pointwise scale is folded into b's
-// twist as in launch_transforms (squarings keep it in the row pass).  With fz
+// twist as in launch_transforms (squarings: into the untwist).  With fz
 // the operands are integer polynomials (an, bn coefficients).
 static void launch_transforms3(const Ctx *X, int np, int k, int logMs, const uint64_t *a, uint64_t an,
                                const uint64_t *b, uint64_t bn, uint32_t *ra, uint32_t *rb, bool sq,
@@ -1242,10 +1267,11 @@ static void launch_transforms3(const Ctx *X, int np, int k, int logMs, const uin
                X->T, a, an, b, bn, ra, rb, logMs, k, sc, sq ? 0 : 2, fz ? *fz : FzShape{1, 1, 1});
     timing_mark(tr, 1, st);
     const LaunchShape L = make_shape(logMs, LOGC3);   // row launch shape (one 2^13-point row per item)
-    launch_rows(X, L, 5, ra, rb, logMs - LOGC3, np, sq ? sc : nullptr, sq ? 1 : 0, nullptr, 1, rows, st,
+    launch_rows(X, L, 5, ra, rb, logMs - LOGC3, np, nullptr, sq ? 1 : 0, nullptr, 1, rows, st,
                 rows_dependent((size_t)3 << k, LOGC3));
     timing_mark(tr, 2, st);
-    launch_dep(INV_COLS3[r - LOG3_RMIN], dim3(C / G, np), THREADS3, smem, st, true, X->T, ra, logMs, k);
+    launch_dep(INV_COLS3[r - LOG3_RMIN + (sq ? 6 : 0)], dim3(C / G, np), THREADS3, smem, st, true, X->T, ra, logMs, k,
+               sq ? sc : nullptr);
     timing_mark(tr, 3, st);
 }
 
@@ -1478,7 +1504,7 @@ static int mpn_mul_enqueue(Ctx *X, uint64_t *z, const uint64_t *a, uint64_t an,
         const FzShape one{1, 1, 1};
         if (b_ready) CU(cudaStreamWaitEvent(st, b_ready, 0));
         fwd_cols_kernel(S.logR, S.logC)<<<dim3(np, Ls.col_grid, 1), Ls.col_threads, Ls.col_smem, st>>>(
-            X->T, y, yn, y, yn, cb, cb, S.logC, S.G, nullptr, np, one, nullptr, 0);
+            X->T, y, yn, y, yn, cb, cb, S.logC, S.G, nullptr, np, one, scale_ptr(X, np, Lc), 1);   // y carries the scale
         ROWS_FWD[S.logC]<<<((1 << S.logR) / Ls.nv) * np, Ls.nv * (1 << S.logC) / 32,
                            Ls.nv * padw(1 << S.logC) * sizeof(uint32_t), st>>>(X->T, cb, S.logR, Ls.nv, np,
                                                                               1 << S.logR);
@@ -1488,9 +1514,9 @@ static int mpn_mul_enqueue(Ctx *X, uint64_t *z, const uint64_t *a, uint64_t an,
             const ChunkOut co{ra, logM, i * c, i ? yn - 1 : 0, xi + yn - 1};
             fwd_cols_kernel(S.logR, S.logC)<<<dim3(np, Ls.col_grid, 1), Ls.col_threads, Ls.col_smem, st>>>(
                 X->T, x + i * c, xi, x + i * c, xi, ca, ca, S.logC, S.G, nullptr, np, one, nullptr, 0);
-            launch_rows(X, Ls, 5, ca, cb, S.logR, np, scale_ptr(X, np, Lc), 2, nullptr, 1, 1 << S.logR, st, false);
+            launch_rows(X, Ls, 5, ca, cb, S.logR, np, nullptr, 2, nullptr, 1, 1 << S.logR, st, false);
             inv_cols_kernel(S.logR, S.logC)<<<dim3(Ls.col_grid, np, 1), Ls.col_threads, Ls.col_smem, st>>>(X->T, ca, S.logC, S.G,
-                                                                                          nullptr, co);
+                                                                                          nullptr, co, nullptr);
             launches += 3;
         }
         timing_mark(tr, 1, st);

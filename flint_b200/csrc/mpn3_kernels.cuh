@@ -270,9 +270,9 @@ k_fwd_cols3(DevTables T, const uint64_t* __restrict__ a, uint64_t an, const uint
 // Inverse column pass of a 3 2^k-point transform, in place: untwist, three
 // length-2^LOGR inverse transforms, inverse radix-3 stage.
 // grid = (C / G, np); block THREADS3; smem as k_fwd_cols3.
-template <int LOGR, int G>
+template <int LOGR, int G, bool SC = false>
 __global__ void __launch_bounds__(THREADS3, CTAS3)
-k_inv_cols3(DevTables T, uint32_t* __restrict__ ra, int logMs, int k)
+k_inv_cols3(DevTables T, uint32_t* __restrict__ ra, int logMs, int k, const uint32_t* __restrict__ fscale)
 {
     extern __shared__ uint32_t sm[];
     constexpr int RP = 1 << LOGR;
@@ -282,6 +282,8 @@ k_inv_cols3(DevTables T, uint32_t* __restrict__ ra, int logMs, int k)
     uint32_t* __restrict__ buf = ra + ((size_t)j << logMs);
     const PrimeInfo P = T.pi[j];
     const uint32_t p = P.p;
+    uint32_t fsc = 0;                    // SC: as in k_inv_cols
+    if constexpr (SC) fsc = fscale[j];
     const uint2* __restrict__ th3 = T.th3i + (size_t)j * TH3_SZ;
     const uint2* __restrict__ tl3 = T.tl3i + (size_t)j * TL_SZ;
     constexpr int NS = RP / 32;
@@ -295,7 +297,7 @@ k_inv_cols3(DevTables T, uint32_t* __restrict__ ra, int logMs, int k)
         uint32_t xr[32];
 #pragma unroll
         for (int m = 0; m < 32; m++) xr[m] = src[m * C];
-        twist32_3<LOGR>(xr, col, s, t, k, th3, tl3, P, 0u);
+        twist32_3<LOGR>(xr, col, s, t, k, th3, tl3, P, fsc);
         ct_contig<5, COL_CT_FMA_ADDS>(xr, c_w32[j], p);
         const int pb = padw(t * RP * G) + 33 * G * s + v;
 #pragma unroll

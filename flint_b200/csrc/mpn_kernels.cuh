@@ -672,9 +672,9 @@ k_rows(DevTables T, uint32_t* __restrict__ ra, const uint32_t* __restrict__ rb,
                 xr[m] = mul_mont(mul_mont(xr[m], y, p, P.pneg_inv), sc, p, P.pneg_inv);
             }
         } else {
-            // the scale was folded into b's forward transform (k_fwd_cols)
+            // the scale was folded into a column pass (or a ring product's untwist)
 #pragma unroll
-            for (int m = 0; m < E; m++) xr[m] = mul_mont(xr[m], breg[m], p, P.pneg_inv);
+            for (int m = 0; m < E; m++) xr[m] = mul_mont(xr[m], squaring == 1 ? xr[m] : breg[m], p, P.pneg_inv);
         }
         ct_contig<LOGE, ROW_CT_FMA_ADDS>(xr, c_w32[j], p);
 #pragma unroll
@@ -804,10 +804,13 @@ struct ChunkOut {
 // ---------------------------------------------------------------------------
 // Column pass, inverse: untwist in registers + length-R inverse transforms,
 // in place (or into a split product's residues, ChunkOut).  grid = (C / G, np, instances); smem = padw(R * G) words.
-template <int LOGR, int G, int LC>
+// SC: the pointwise scale folded into the untwist (squarings; as instances of
+// their own, since the run-time choice cost the others 6%: 2^10-point columns
+// 120.8 -> 128.3 us).
+template <int LOGR, int G, int LC, bool SC>
 __device__ __forceinline__ void
 inv_cols_body(DevTables T, uint32_t* __restrict__ ra, int logC, int gcols,
-              const InstDesc* __restrict__ desc, ChunkOut co)
+              const InstDesc* __restrict__ desc, ChunkOut co, const uint32_t* __restrict__ fscale)
 {
     extern __shared__ uint32_t sm[];
     constexpr int R = 1 << LOGR;
@@ -816,6 +819,8 @@ inv_cols_body(DevTables T, uint32_t* __restrict__ ra, int logC, int gcols,
     const int logM = LOGR + logC;
     const int GR = G ? G : gcols;
     const int j = blockIdx.y;
+    uint32_t fsc = 0;
+    if constexpr (SC) fsc = fscale[j];
     const int i0 = blockIdx.x * GR;
     if (desc) ra = desc[blockIdx.z].ra;
     uint32_t* __restrict__ buf = ra + ((size_t)j << logM);
@@ -841,7 +846,7 @@ inv_cols_body(DevTables T, uint32_t* __restrict__ ra, int logC, int gcols,
             const uint32_t* src = buf + ((size_t)(32 * s) << logC) + col;
 #pragma unroll
             for (int m = 0; m < 32; m++) xr[m] = src[(size_t)m * C];
-            twist32<LOGR>(xr, col, s, logM, th, tl, P);
+            twist32<LOGR>(xr, col, s, logM, th, tl, P, fsc);
             ct_contig<5, COL_CT_FMA_ADDS>(xr, c_w32[j], p);
             if constexpr (LOGR == 5) {
                 // the whole column is in registers
@@ -890,17 +895,17 @@ inv_cols_body(DevTables T, uint32_t* __restrict__ ra, int logC, int gcols,
     }
 }
 
-template <int LOGR, int G, int LC = 0>
+template <int LOGR, int G, int LC = 0, bool SC = false>
 __global__ void __launch_bounds__(512)
 k_inv_cols(DevTables T, uint32_t* __restrict__ ra, int logC, int gcols,
-           const InstDesc* __restrict__ desc, ChunkOut co)
+           const InstDesc* __restrict__ desc, ChunkOut co, const uint32_t* __restrict__ fscale)
 {
     // as the forward pass: the constant-stride instances serve large products
     if constexpr (LC == 0) {
         pdl_wait();
         pdl_trigger();
     }
-    inv_cols_body<LOGR, G, LC>(T, ra, logC, gcols, desc, co);
+    inv_cols_body<LOGR, G, LC, SC>(T, ra, logC, gcols, desc, co, fscale);
 }
 
 // ---------------------------------------------------------------------------

@@ -10,10 +10,9 @@
 //
 //   k_neg_split     digit i -> residue, times omega^i        [per prime]
 //   k_rows          length-m forward transforms of x and y, pointwise product
-//                   with 2^128 / m, inverse transform (the mpn row kernel, one
-//                   row per product)
+//                   inverse transform (the mpn row kernel, one row per product)
 //   k_neg_finish    per product: untwist omega^-i with the CRT cofactor
-//                   inverse, add a bias B = 2^(2b + log m) so every coefficient
+//                   inverse and the normalisation 2^128 / m, add a bias B = 2^(2b + log m) so every coefficient
 //                   is non-negative, CRT, recompose sum V_i 2^(b i) with the
 //                   carries, add (-biaspoly mod 2^N + 1), fold mod 2^N + 1.
 //
@@ -84,11 +83,10 @@ __global__ void k_neg_split(DevTables T, const uint64_t* __restrict__ x, uint32_
     }
 }
 
-// X <- X F scale_k 2^-64 (the fused row pass's pointwise normalisation) on
-// rows 0 .. count-1 of every prime; X and F share the layout of k_neg_split.
+// X <- X F 2^-32 (the fused row pass's pointwise product; the untwist carries the
+// normalisation) on rows 0 .. count-1 of every prime; X and F share the layout of k_neg_split.
 __global__ void k_neg_pointwise(DevTables T, uint32_t* __restrict__ X, const uint32_t* __restrict__ F,
-                                uint32_t count, int logm, int logR, int np,
-                                const uint32_t* __restrict__ scale)
+                                uint32_t count, int logm, int logR, int np)
 {
     const uint64_t per = (uint64_t)count << logm;
     const uint64_t total = per * np;
@@ -99,7 +97,7 @@ __global__ void k_neg_pointwise(DevTables T, uint32_t* __restrict__ X, const uin
         const int k = (int)(e / per);
         const size_t idx = ((size_t)k << (logR + logm)) + (e - (uint64_t)k * per);
         const PrimeInfo& P = T.pi[k];
-        X[idx] = mul_mont(mul_mont(X[idx], F[idx], P.p, P.pneg_inv), scale[k], P.p, P.pneg_inv);
+        X[idx] = mul_mont(X[idx], F[idx], P.p, P.pneg_inv);
     }
 }
 
@@ -162,7 +160,7 @@ __device__ __forceinline__ bool neg_block_carry_in(bool g, bool p, uint32_t* s_w
 
 // One CTA per product: untwist, bias, CRT, recomposition, fold.
 // buf: residues after the inverse transforms (natural order, layout of
-// k_neg_split); itw holds omega^-i (P/p_k)^-1 2^32 mod p_k; beta holds
+// k_neg_split); itw holds omega^-i (P/p_k)^-1 2^128 / m mod p_k; beta holds
 // (-sum_i B 2^(b i)) mod 2^N + 1 in n + 1 limbs.  Dynamic shared memory:
 // 3 NEG_CMAX 64-bit words.
 template <int NP>
