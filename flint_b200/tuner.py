@@ -76,12 +76,13 @@ def candidates(r, flags=True):
         for dm in (0, 1):
             np_, logM = base.np + dnp, base.logM + dm
             # the rule's row length for this length, then the longest rows
-            # and 2x / 4x / 8x shorter
+            # and 2x / 4x / 8x shorter, and the short rows that planned
+            # batches take by themselves (2^9 points, 2^11 at 2^19)
             try:
                 rule_logC = [resolve_config(kind, an, bn, MulConfig(ROUTE_NTT, np_, logM, 0), aw, bw).logC]
             except GpuFftSmallError:
                 rule_logC = []
-            for logC in rule_logC + [min(logM, 14) - dc for dc in (0, 1, 2, 3)]:
+            for logC in rule_logC + [min(logM, 14) - dc for dc in (0, 1, 2, 3)] + ([9, 11] if logM >= 14 else []):
                 if (np_, logM, logC) in seen:
                     continue
                 seen.add((np_, logM, logC))

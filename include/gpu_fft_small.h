@@ -387,8 +387,10 @@ GPU_FFT_SMALL_API int gpu_mulmod_2expp1_mul_cached(const gpu_mulmod_2expp1_ctx_s
    primes that hold the coefficient bound, the shortest transform that holds
    the product, rows of 2^logM points up to 2^13, 32-point columns from 2^14
    to 2^17 points, 64-point columns at 2^18, 2^13-point rows from 2^19 to
-   2^24 points, 2^14 at 2^25.  Any valid choice gives the same (exact)
-   product; only the time differs. */
+   2^24 points, 2^14 at 2^25.  (A product without a configuration, and a
+   planned batch's request that leaves logC 0, take row lengths fitted to the
+   kernels instead.)  Any valid choice gives the same (exact) product; only
+   the time differs. */
 typedef struct {
     int route;   /* GPU_MUL_ROUTE_* */
     int np;      /* primes, minimal .. 6 */
