@@ -116,6 +116,7 @@ SIGNATURES = {
     "gpu_mpn_pipe_submit": (ctypes.c_int, [_PIPE, _P, _P, _U, _P, _U, ctypes.POINTER(ctypes.c_longlong)]),
     "gpu_mpn_pipe_wait": (ctypes.c_int, [_PIPE, ctypes.c_longlong]),
     "gpu_mpn_pipe_clear": (None, [_PIPE]),
+    "gpu_mpn_ctx_check": (ctypes.c_int, [_CTX, _P]),
     "gpu_test_crt_lookback_timeout": (ctypes.c_int, [_CTX]),
     "gpu_test_set_device_error": (ctypes.c_int, [_CTX]),
     "gpu_test_pipe_slot_ctx": (ctypes.c_void_p, [_PIPE, ctypes.c_int]),
@@ -517,6 +518,10 @@ class MpnCtx:
                                               ctypes.byref(cfg) if cfg is not None else None,
                                               copies, reps, ctypes.byref(ms)))
         return ms.value
+
+    def check(self, stream=None):
+        """Wait for `stream`; raises if a kernel of the context's device-pointer calls recorded an error."""
+        _check(lib().gpu_mpn_ctx_check(self.ptr, stream))
 
     def nmod_poly_divrem(self, a, b, n):
         """(q, r) with a = q b + r mod n, deg r < deg b (_nmod_poly_divrem_mpn_ctx)."""

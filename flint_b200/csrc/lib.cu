@@ -1550,16 +1550,22 @@ static int mpn_mul_enqueue(Ctx *X, uint64_t *z, const uint64_t *a, uint64_t an,
     return 0;
 }
 
+// The error flag as *X->h_err holds it: reported and cleared.
+static int take_device_error(Ctx *X)
+{
+    if (!*X->h_err) return 0;
+    *X->h_err = 0;
+    cudaMemsetAsync(X->d_err, 0, sizeof(int), X->stream);
+    return set_error(GPU_FFT_SMALL_ETIMEOUT, "carry look-back wait exceeded its limit");
+}
+
+// Waits for the context's stream and reads the error flag its kernels left
+// (through the pinned word: one copy, no staging).
 static int check_device_error(Ctx *X)
 {
-    int err = 0;
-    CU(cudaMemcpyAsync(&err, X->d_err, sizeof(int), cudaMemcpyDeviceToHost, X->stream));
+    CU(cudaMemcpyAsync(X->h_err, X->d_err, sizeof(int), cudaMemcpyDeviceToHost, X->stream));
     CU(cudaStreamSynchronize(X->stream));
-    if (err) {
-        cudaMemsetAsync(X->d_err, 0, sizeof(int), X->stream);
-        return set_error(GPU_FFT_SMALL_ETIMEOUT, "carry look-back wait exceeded its limit");
-    }
-    return 0;
+    return take_device_error(X);
 }
 
 static int io_buffers(Ctx *X, size_t words, uint64_t **p)
@@ -1689,11 +1695,8 @@ static int mpn_mul_host_finish(Ctx *X, gpu_ulong *z, gpu_ulong an, gpu_ulong bn,
     else if (X->copy_stream) CU(cudaStreamSynchronize(X->copy_stream));
     if (an + bn > lo && std::min<gpu_ulong>(hi, an + bn) > lo) {
         // the flag was copied behind the last download
-        if (*X->h_err) {
-            *X->h_err = 0;
-            cudaMemsetAsync(X->d_err, 0, sizeof(int), X->stream);
-            return set_error(GPU_FFT_SMALL_ETIMEOUT, "carry look-back wait exceeded its limit");
-        }
+        rc = take_device_error(X);
+        if (rc) return rc;
     } else {
         rc = check_device_error(X);
         if (rc) return rc;
@@ -2037,6 +2040,16 @@ int gpu_mpn_mul_device_config(gpu_mpn_ctx_t R, uint64_t *z_dev, const uint64_t *
     int rc = bind_device(X);
     if (rc) return rc;
     return mpn_mul_enqueue(X, z_dev, a_dev, an, b_dev, bn, (cudaStream_t)stream, cfg);
+}
+
+int gpu_mpn_ctx_check(gpu_mpn_ctx_t R, void *stream)
+{
+    Ctx *X = get_ctx(R);
+    if (!X) return set_error(GPU_FFT_SMALL_EINVAL, "context not initialised");
+    int rc = bind_device(X);
+    if (rc) return rc;
+    CU(cudaStreamSynchronize((cudaStream_t)stream));
+    return check_device_error(X);
 }
 
 int gpu_mpn_mul_range_device(gpu_mpn_ctx_t R, uint64_t *z_dev, gpu_ulong lo, gpu_ulong hi,

@@ -149,6 +149,14 @@ GPU_FFT_SMALL_API int gpu_mpn_mul_device(gpu_mpn_ctx_t R, uint64_t *z_dev,
                        const uint64_t *a_dev, gpu_ulong an,
                        const uint64_t *b_dev, gpu_ulong bn, void *stream);
 
+/* Waits for `stream` and reports a kernel error of the context's device-pointer
+   calls (a bounded wait that gave up), as gpu_mpn_batch_check and
+   gpu_fft_op_check do for theirs: GPU_FFT_SMALL_ETIMEOUT if any kernel of the
+   context recorded one since the last check, else 0.  Host-pointer calls check
+   by themselves, so an error left unread fails the next of them.  (No
+   counterpart in the reference, whose calls return with the product done.) */
+GPU_FFT_SMALL_API int gpu_mpn_ctx_check(gpu_mpn_ctx_t R, void *stream);
+
 /* Allocation-free product on device pointers (no counterpart in the
    reference).  For callers that cannot call cudaMalloc: a framework that owns
    all device memory through its own pool and forbids outside allocations, or
@@ -481,7 +489,7 @@ GPU_FFT_SMALL_API int gpu_fmpz_poly_mul_mid_device_list(gpu_mpn_ctx_t R, const g
    flag and finishes; returns the status the host reads back
    (GPU_FFT_SMALL_ETIMEOUT) and leaves the context usable.
    gpu_test_set_device_error sets the error flag as such a kernel would: the
-   next host-pointer product on the context returns GPU_FFT_SMALL_ETIMEOUT
+   next host-pointer call on the context returns GPU_FFT_SMALL_ETIMEOUT
    and clears it.  gpu_test_pipe_slot_ctx returns the context behind slot
    `slot` of a pipeline (the impl of a gpu_mpn_ctx_t), or NULL. */
 GPU_FFT_SMALL_API int gpu_test_crt_lookback_timeout(gpu_mpn_ctx_t R);
@@ -693,7 +701,7 @@ GPU_FFT_SMALL_API int gpu_fft_export_mpn_signed(uint64_t *z_dev, gpu_ulong zn, i
 GPU_FFT_SMALL_API int gpu_fft_export_mpn_signed_trunc(uint64_t *z_dev, gpu_ulong zn, int *sign, gpu_fft_op_t X,
                                                       gpu_ulong nslots, gpu_ulong lo_limbs, gpu_fft_plan_t P,
                                                       void *stream);
-/* Synchronises `stream`; GPU_FFT_SMALL_ETIMEOUT if a carry wait gave up. */
+/* Synchronises `stream`; GPU_FFT_SMALL_ETIMEOUT if a bounded wait gave up. */
 GPU_FFT_SMALL_API int gpu_fft_op_check(gpu_fft_plan_t P, void *stream);
 
 /* --- batches of uneven products (no counterpart in the reference, which
