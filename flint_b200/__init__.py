@@ -119,6 +119,7 @@ SIGNATURES = {
     "gpu_mpn_ctx_check": (ctypes.c_int, [_CTX, _P]),
     "gpu_test_crt_lookback_timeout": (ctypes.c_int, [_CTX]),
     "gpu_test_set_device_error": (ctypes.c_int, [_CTX]),
+    "gpu_test_set_device_error_bits": (ctypes.c_int, [_CTX, ctypes.c_int]),
     "gpu_test_pipe_slot_ctx": (ctypes.c_void_p, [_PIPE, ctypes.c_int]),
     "_gpu_mpn_ctx_mpn_mul_range": (None, [_CTX, _P, _U, _U, _P, _U, _P, _U]),
     "gpu_mpn_mul_device": (ctypes.c_int, [_CTX, _P, _P, _U, _P, _U, _P]),

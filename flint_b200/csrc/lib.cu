@@ -1553,10 +1553,16 @@ static int mpn_mul_enqueue(Ctx *X, uint64_t *z, const uint64_t *a, uint64_t an,
 // The error flag as *X->h_err holds it: reported and cleared.
 static int take_device_error(Ctx *X)
 {
-    if (!*X->h_err) return 0;
+    const int err = *X->h_err;
+    if (!err) return 0;
     *X->h_err = 0;
     cudaMemsetAsync(X->d_err, 0, sizeof(int), X->stream);
-    return set_error(GPU_FFT_SMALL_ETIMEOUT, "carry look-back wait exceeded its limit");
+    if (err & DEV_ERR_ALIGN)
+        return set_error(GPU_FFT_SMALL_ECUDA, "row pass: shared memory not aligned for the operand tiles");
+    return set_error(GPU_FFT_SMALL_ETIMEOUT, "%s",
+                     !(err & DEV_ERR_ROWS)    ? "carry look-back wait exceeded its limit"
+                     : !(err & DEV_ERR_CARRY) ? "row pass: wait for a matrix product exceeded its limit"
+                                              : "row pass and carry look-back waits exceeded their limits");
 }
 
 // Waits for the context's stream and reads the error flag its kernels left
@@ -2296,16 +2302,18 @@ void *gpu_test_pipe_slot_ctx(gpu_mpn_pipe_t R, int slot)
     return P->slot[slot];
 }
 
-int gpu_test_set_device_error(gpu_mpn_ctx_t R)
+int gpu_test_set_device_error_bits(gpu_mpn_ctx_t R, int bits)
 {
     Ctx *X = get_ctx(R);
     if (!X) return set_error(GPU_FFT_SMALL_EINVAL, "context not initialised");
     int rc = bind_device(X);
     if (rc) return rc;
-    CU(cudaMemsetAsync(X->d_err, 1, sizeof(int), X->stream));
+    CU(cudaMemcpyAsync(X->d_err, &bits, sizeof(int), cudaMemcpyHostToDevice, X->stream));
     CU(cudaStreamSynchronize(X->stream));
     return 0;
 }
+
+int gpu_test_set_device_error(gpu_mpn_ctx_t R) { return gpu_test_set_device_error_bits(R, DEV_ERR_CARRY); }
 
 int gpu_butterfly_rate(gpu_mpn_ctx_t R, double *per_s)
 {

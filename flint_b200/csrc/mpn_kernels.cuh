@@ -56,8 +56,13 @@ struct DevTables {
     const uint2* w3c;      // [NP3][2] (w - w^2, w^-1 - w^-2), w = w3^(2^25) of order 3
     const uint4* tcw;      // [MAX_NP] swizzled W images (tc_fill_w), TC_W_BYTES each
     const TcPrime* tcp;    // [MAX_NP]
-    int* err;              // the context's device error flag
+    int* err;              // the context's device error flag (DEV_ERR_*)
 };
+
+// Bits of a context's error flag, set by kernels whose results are not valid.
+constexpr int DEV_ERR_CARRY = 1;   // a carry look-back gave up waiting
+constexpr int DEV_ERR_ROWS = 2;    // the row pass gave up waiting for a matrix product
+constexpr int DEV_ERR_ALIGN = 4;   // the row pass found its operand tiles misaligned
 
 // Programmatic dependent launch.  A kernel launched as a programmatic
 // dependent (launch_dep in lib.cu) may start while its predecessor on the
@@ -1270,7 +1275,7 @@ k_crt_carry(const uint32_t* __restrict__ res, int logM, uint64_t L, uint64_t zn,
             while (true) {
                 const uint32_t st = *(volatile uint32_t*)&status[k];
                 if ((st >> 4) != epoch || (st & (3u << 2)) == 0) {
-                    if (++spins > LOOKBACK_SPIN_LIMIT) { atomicExch(err, 1); cin = 0; break; }
+                    if (++spins > LOOKBACK_SPIN_LIMIT) { atomicOr(err, DEV_ERR_CARRY); cin = 0; break; }
                     __nanosleep(64);
                     continue;
                 }

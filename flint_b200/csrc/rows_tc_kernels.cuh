@@ -185,7 +185,8 @@ k_rows_tc(DevTables T, uint32_t* __restrict__ ra, const uint32_t* __restrict__ r
     // the operand tiles need 1024-byte alignment, which dynamic shared memory
     // has here (the kernel has no static one)
     if (tc_smem(sm) & 1023u) {
-        if (t == 0) atomicExch(T.err, 1);
+        pdl_wait();   // the grid must not end before the kernel it follows
+        if (t == 0) atomicOr(T.err, DEV_ERR_ALIGN);
         return;
     }
     if (t < 32) tc_alloc(tc_smem(taddr), TC_COLS);
@@ -223,7 +224,7 @@ k_rows_tc(DevTables T, uint32_t* __restrict__ ra, const uint32_t* __restrict__ r
         }
         if (!dead && !tc_mbar_wait(bar_s, phase)) {   // never on a working device: flag it and finish
             dead = true;
-            atomicExch(T.err, 1);
+            atomicOr(T.err, DEV_ERR_ROWS);
         }
         phase ^= 1;
         tc_fence_after();

@@ -490,10 +490,14 @@ GPU_FFT_SMALL_API int gpu_fmpz_poly_mul_mid_device_list(gpu_mpn_ctx_t R, const g
    (GPU_FFT_SMALL_ETIMEOUT) and leaves the context usable.
    gpu_test_set_device_error sets the error flag as such a kernel would: the
    next host-pointer call on the context returns GPU_FFT_SMALL_ETIMEOUT
-   and clears it.  gpu_test_pipe_slot_ctx returns the context behind slot
+   and clears it.  gpu_test_set_device_error_bits sets the bits a kernel would:
+   1 a carry look-back (as the former), 2 a row pass's wait for a matrix product
+   (both GPU_FFT_SMALL_ETIMEOUT, each with its own message), 4 a row pass whose
+   shared memory is misaligned (GPU_FFT_SMALL_ECUDA).  gpu_test_pipe_slot_ctx returns the context behind slot
    `slot` of a pipeline (the impl of a gpu_mpn_ctx_t), or NULL. */
 GPU_FFT_SMALL_API int gpu_test_crt_lookback_timeout(gpu_mpn_ctx_t R);
 GPU_FFT_SMALL_API int gpu_test_set_device_error(gpu_mpn_ctx_t R);
+GPU_FFT_SMALL_API int gpu_test_set_device_error_bits(gpu_mpn_ctx_t R, int bits);
 GPU_FFT_SMALL_API void *gpu_test_pipe_slot_ctx(gpu_mpn_pipe_t P, int slot);
 
 /* Integer-pipe calibration (no counterpart in the reference): the rate, in
@@ -756,7 +760,7 @@ GPU_FFT_SMALL_API int gpu_mpn_batch_init_config(gpu_mpn_batch_t *B, gpu_mpn_ctx_
                                                 size_t n, const gpu_mpn_batch_options *opt);
 /* Queues every product of the batch on `stream` (NULL = CUDA's default
    stream) and returns without synchronising.  Runs of one batch must not
-   overlap.  Kernel errors (a carry look-back that gave up) are reported by
+   overlap.  Kernel errors (a bounded wait that gave up) are reported by
    gpu_mpn_batch_check. */
 GPU_FFT_SMALL_API int gpu_mpn_batch_run(gpu_mpn_batch_t B, void *stream);
 /* Waits for `stream` and returns GPU_FFT_SMALL_ETIMEOUT if any kernel of the

@@ -65,3 +65,16 @@ def test_device_calls_have_a_check(ctx):
         ctx.check(s)
     assert e.value.code == FB.ETIMEOUT
     ctx.check(s)
+
+
+@pytest.mark.parametrize("bits,code,words", [(1, "ETIMEOUT", ["carry"]), (2, "ETIMEOUT", ["row pass", "matrix product"]),
+                                             (3, "ETIMEOUT", ["row pass", "carry"]), (4, "ECUDA", ["row pass", "aligned"])])
+def test_message_names_the_kernel(ctx, bits, code, words):
+    """The row pass's errors are not reported as the carry look-back's."""
+    FB._check(FB.lib().gpu_test_set_device_error_bits(ctx.ptr, bits))
+    with pytest.raises(FB.GpuFftSmallError) as e:
+        ctx.mpn_mul(O.rand_limbs(1, 100), O.rand_limbs(2, 100))
+    assert e.value.code == getattr(FB, code)
+    assert all(w in str(e.value) for w in words)
+    assert ("carry" in str(e.value)) == bool(bits & 1)
+    ctx.check()
