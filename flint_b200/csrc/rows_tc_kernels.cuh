@@ -222,10 +222,13 @@ k_rows_tc(DevTables T, uint32_t* __restrict__ ra, const uint32_t* __restrict__ r
             tc_mma_tile(tm + 128, tc_smem(buf) + TC_TILE_BYTES, tc_smem(sw));
             tc_commit(bar_s);
         }
-        if (!dead && !tc_mbar_wait(bar_s, phase)) {   // never on a working device: flag it and finish
-            dead = true;
+        // a warp gives up as one, and is converged again (thread 0's branch, each
+        // thread's own polls) before the aligned loads that follow
+        if (!dead && !__all_sync(0xffffffffu, tc_mbar_wait(bar_s, phase))) {
+            dead = true;                              // never on a working device: flag it and finish
             atomicOr(T.err, DEV_ERR_ROWS);
         }
+        __syncwarp();
         phase ^= 1;
         tc_fence_after();
     };

@@ -47,3 +47,16 @@ def test_tensor_loads_end_with_their_wait(path):
 def test_the_row_pass_has_such_loads():
     text = "".join(open(p).read() for p in files())
     assert any("tcgen05.ld" in s for s in asm_statements(text))
+
+
+@pytest.mark.parametrize("path", files(), ids=os.path.basename)
+def test_warps_converge_after_a_polled_wait(path):
+    """tcgen05's .sync.aligned instructions need the whole warp together; a loop
+    of polls that each thread leaves by itself does not bring it there, so a
+    warp-wide decision and a __syncwarp stand between the poll and what follows."""
+    text = re.sub(r"//[^\n]*", "", open(path).read())
+    for m in re.finditer(r"(?<!bool )\btc_mbar_wait\s*\(", text):
+        line = text[text.rindex("\n", 0, m.start()):m.start()]
+        assert re.search(r"__(all|any)_sync\s*\(\s*0xffffffffu\s*,\s*!?$", line), line
+        rest = text[m.end():]
+        assert "__syncwarp()" in rest[:rest.index("tc_fence_after()")]
