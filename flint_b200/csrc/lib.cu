@@ -741,13 +741,13 @@ static bool rows_dependent(size_t points, int logC, int loge = 5)
 // with fz the operands are integer polynomials (an, bn coefficients); with co
 // the inverse column pass writes a split product's chunk (ChunkOut).  Returns
 // the residue array that holds the product (ra, or rb for a large product
-// whose b arrives late: b_ready)
+// whose b arrives late: b_ready); *launches is set to the kernels launched
 static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, const uint64_t *a,
                               uint64_t an, const uint64_t *b, uint64_t bn, uint32_t *ra,
                               uint32_t *rb, bool sq, const uint32_t *d_scale, cudaStream_t st,
                               TimingRecord *tr, const InstDesc *desc = nullptr, int ninst = 1,
                               const FzShape *fz = nullptr, cudaEvent_t b_ready = nullptr,
-                              const ChunkOut *co = nullptr);
+                              const ChunkOut *co = nullptr, int *launches = nullptr);
 
 static int upload_scales(Ctx *X);
 
@@ -1169,9 +1169,14 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
                                    uint64_t an, const uint64_t *b, uint64_t bn, uint32_t *ra,
                                    uint32_t *rb, bool sq, const uint32_t *d_scale, cudaStream_t st,
                                    TimingRecord *tr, const InstDesc *desc, int ninst, const FzShape *fz,
-                                   cudaEvent_t b_ready, const ChunkOut *co)
+                                   cudaEvent_t b_ready, const ChunkOut *co, int *launches)
 {
     const MulShape &S = L.S;
+    int nl = S.logR > 0 ? 3 : 2;   // forward columns (or the split alone), rows, inverse columns
+    auto done = [&](uint32_t *r) {
+        if (launches) *launches = nl;
+        return r;
+    };
     const int zdim = desc ? 2 * ninst : (sq ? 1 : 2);
     const int ni = desc ? ninst : 1;
     const ColLaunch cf = col_launch(X, L, np, zdim, fz != nullptr);
@@ -1199,9 +1204,11 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
                    (sq && !desc) ? 1 : 0, desc, shape);
         timing_mark(tr, 2, st);
         timing_mark(tr, 3, st);
-        return ra;
+        nl = 1;
+        return done(ra);
     }
     if (b_ready && !desc && !sq) {
+        nl++;                      // a column launch for each operand
         // b is still arriving: a's column pass first, b's after its copy
         fwd<<<dim3(np, cf.grid, 1), cf.threads, cf.smem, st>>>(X->T, a, an, a, an, ra, ra, S.logC, cf.G, nullptr,
                                                                np, shape, d_scale, 0);
@@ -1215,6 +1222,7 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
             const int C = 1 << S.logC, groups = (R + L.nv - 1) / L.nv;
             ROWS_FWD[S.logC]<<<groups * np, L.nv * C / 32, (size_t)L.nv * padw(C) * sizeof(uint32_t), st>>>(
                 X->T, ra, S.logR, L.nv, np, R);
+            nl++;
         }
         cudaStreamWaitEvent(st, b_ready, 0);
         const FzShape shb = fz ? FzShape{shape.S, shape.wb, shape.wb} : shape;
@@ -1227,7 +1235,7 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
             inv<<<dim3(ci.grid, np, 1), ci.threads, ci.smem, st>>>(X->T, rb, S.logC, ci.G, nullptr,
                                                                    ChunkOut{nullptr, 0, 0, 0, 0}, nullptr);
             timing_mark(tr, 3, st);
-            return rb;
+            return done(rb);
         }
     } else {
         if (b_ready) cudaStreamWaitEvent(st, b_ready, 0);
@@ -1244,7 +1252,7 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
         launch_dep(inv, dim3(ci.grid, np, ni), ci.threads, ci.smem, st, dep && S.logR < 9, X->T, ra, S.logC, ci.G, desc,
                    co ? *co : ChunkOut{nullptr, 0, 0, 0, 0}, fold_inv ? d_scale : nullptr);
     timing_mark(tr, 3, st);
-    return ra;
+    return done(ra);
 }
 
 // Transform of M = 3 2^k points (k - 13 in [LOG3_RMIN, LOG3_RMAX]): columns of
@@ -1527,7 +1535,7 @@ static int mpn_mul_enqueue(Ctx *X, uint64_t *z, const uint64_t *a, uint64_t an,
     } else {
         // the product's residues: ra, or rb when b arrived late (launch_transforms)
         ra = launch_transforms(X, P.L, np, a, an, b, bn, ra, rb, sq, scale_ptr(X, np, logM), st, tr, nullptr, 1,
-                               nullptr, b_ready);
+                               nullptr, b_ready, nullptr, &launches);
     }
     // tiles take their index from the ticket counter, so consecutive launches
     // with the same ticket base continue one carry chain: tile k's look-back
@@ -1539,10 +1547,10 @@ static int mpn_mul_enqueue(Ctx *X, uint64_t *z, const uint64_t *a, uint64_t an,
         launch_dep(np == 5 ? k_crt_carry<5, THREADS> : k_crt_carry<6, THREADS>, t1 - t0, THREADS, 0, st, nch == 1,
                    ra, logM, an + bn - 1, zn, z, K, X->d_status, X->d_ticket, X->ticket_base, X->epoch, X->d_err,
                    nullptr, nullptr, base);
+        launches++;
         if (chunks && chunks->hook)
             chunks->hook(chunks->arg, base + t0 * TILE, std::min<uint64_t>(zn, base + t1 * TILE));
     }
-    launches++;
     timing_mark(tr, 4, st);
     X->ticket_base += tiles;
     X->last_launches = launches;
