@@ -15,7 +15,8 @@ Prints one JSON line (rank 0).  Our arm:
               (CUDA events recorded by the library between launches);
   cpu_baseline the reference's own fft_small (oracle/_ref, compiled from the
               reference tree) timed on this host's cores.
-The reference arm (--impl reference) times that CPU implementation alone.
+The reference arm (--impl reference) times that CPU implementation alone, and
+prints an "unavailable" line where it is not built.
 Under torchrun each rank runs an independent replica (no collective on the
 data path); the device time is the max over ranks.
 """
@@ -870,6 +871,13 @@ def main():
 
     if args.impl == "reference":
         if rank != 0:
+            return
+        import oracle
+        if not oracle.have_ref():
+            # only the reference itself is a reference arm: never the oracle's restatement
+            print(json.dumps({"impl": "reference", "unavailable":
+                              "the compiled reference (oracle/_ref/libflint_ref.so) is not built: "
+                              "no reference source tree here"}), flush=True)
             return
         cb = cpu_baseline_run(an, bn, args.steps, args.warmup, max_seconds=240.0)
         line = {"impl": "reference", "metric": METRIC, "value": cb["value"], "unit": "Gbit/s",
