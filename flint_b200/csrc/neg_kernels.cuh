@@ -53,8 +53,10 @@ __global__ void k_neg_split(DevTables T, const uint64_t* __restrict__ x, uint32_
     const uint32_t m = 1u << sh.logm;
     const uint64_t total = (uint64_t)count << sh.logm;
     const uint32_t b = sh.b;
+    // no early trigger: the row kernel's few CTAs would share SMs that are free a
+    // moment later (500 products mod 2^12288 + 1: 32.8 us plain, 36.2 with a trigger
+    // here, 28.8 without; 64 mod 2^196608 + 1: 59.5, 63.6, 49.2)
     pdl_wait();
-    pdl_trigger();
     for (uint64_t e = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t prod = (uint32_t)(e >> sh.logm), i = (uint32_t)e & (m - 1);

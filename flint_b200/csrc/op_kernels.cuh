@@ -57,7 +57,11 @@ k_rows_fwd(DevTables T, uint32_t* __restrict__ buf, int logR, int nv, int np, in
 }
 
 // inverse row transforms, in place (the normalisation was applied by the
-// pointwise stage); launch shape as k_rows_fwd
+// pointwise stage); launch shape as k_rows_fwd.  No early trigger: the successor
+// may start as row CTAs end.  A ring product's finishing CTAs, one a product,
+// would otherwise gather on the SMs the last row CTAs have left free (100 products
+// mod 2^(2^20) + 1 by kept transforms: 279 us plain, 329 with a trigger at the
+// start, 281 with one before the stores, 250 without; 50: 210, 268, 220, 185).
 template <int LOGC>
 __global__ void __launch_bounds__(512)
 k_rows_inv(DevTables T, uint32_t* __restrict__ buf, int logR, int nv, int np, int rows)
@@ -76,7 +80,6 @@ k_rows_inv(DevTables T, uint32_t* __restrict__ buf, int logR, int nv, int np, in
     const int pb = (t / NSUB) * PC + 33 * (t & (NSUB - 1));
     uint32_t* __restrict__ base = buf + ((size_t)j << logM);
     pdl_wait();
-    pdl_trigger();
     rows_prefetch<LOGC>(sm, base, u0, nv, R);
     cp_async_wait<0>();
     __syncthreads();

@@ -1,0 +1,79 @@
+"""Calls that do less work, or the same work by a given shape, are no slower.
+
+Each test compares two calls timed in turn on one device, the best of several
+runs each, and passes if any of a few attempts is inside its bound; the bounds
+lie midway between the ratio that the placement or shape it guards gives and the
+ratio without it (both in the test's comment).
+"""
+import pytest
+
+import flint_b200 as FB
+
+pytestmark = pytest.mark.gpu
+
+ATTEMPTS = 5
+
+
+def _limbs(torch, *shape):
+    return torch.randint(-(1 << 62), 1 << 62, shape, dtype=torch.int64, device="cuda")
+
+
+def _best(torch, fn, stream, reps):
+    best = float("inf")
+    for _ in range(5):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        with torch.cuda.stream(stream):
+            e0.record()
+            for _ in range(reps):
+                fn()
+            e1.record()
+        torch.cuda.synchronize()
+        best = min(best, e0.elapsed_time(e1))
+    return best
+
+
+def _ratio_below(torch, f, g, bound, reps=30):
+    """time(f) / time(g) < bound in at least one of a few attempts."""
+    stream = torch.cuda.Stream()
+    seen = []
+    for _ in range(ATTEMPTS):
+        ratio = _best(torch, lambda: f(stream.cuda_stream), stream, reps) / \
+            _best(torch, lambda: g(stream.cuda_stream), stream, reps)
+        seen.append(ratio)
+        if ratio < bound:
+            return
+    raise AssertionError("ratios %s, bound %s" % (seen, bound))
+
+
+def _ring(torch, ctx, N, count):
+    C = FB.Mulmod2expp1(ctx, N)
+    n = N // 64
+    x, y, z = (_limbs(torch, count, n + 1) for _ in range(3))
+    x[:, n] = 0
+    y[:, n] = 0
+    return C, x, y, z
+
+
+@pytest.mark.parametrize("count", [50, 64])
+def test_ring_products_by_kept_transforms(ctx, count):
+    """A product by a kept transform does less than a whole one: 1.00-1.02
+    (with finishing CTAs placed beside the inverse rows 1.40-1.48)."""
+    torch = pytest.importorskip("torch")
+    C, x, y, z = _ring(torch, ctx, 1 << 20, count)
+    F = torch.empty(C.transformed_size(count), dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    C.transform_device(F.data_ptr(), y.data_ptr(), count)
+    torch.cuda.synchronize()
+    _ratio_below(torch, lambda s: C.mul_cached_device(z.data_ptr(), x.data_ptr(), F.data_ptr(), count, None, s),
+                 lambda s: C.batch_device(z.data_ptr(), x.data_ptr(), y.data_ptr(), count, None, s), 1.2)
+
+
+@pytest.mark.parametrize("N,count,bound", [(12288, 500, 1.38), (196608, 64, 1.19)])
+def test_ring_products_in_small_numbers(ctx, N, count, bound):
+    """Twice as many products where the GPU is far from full: 1.24 and 1.06 of
+    the time (with row CTAs placed beside the splitting ones 1.52 and 1.31)."""
+    torch = pytest.importorskip("torch")
+    C, x, y, z = _ring(torch, ctx, N, count)
+    torch.cuda.synchronize()
+    run = lambda c: lambda s: C.batch_device(z.data_ptr(), x.data_ptr(), y.data_ptr(), c, None, s)
+    _ratio_below(torch, run(count), run(count // 2), bound)
