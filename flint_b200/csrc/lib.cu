@@ -654,8 +654,8 @@ static int single_logC(int logM)
     if (logM <= 20) return logM - 8;
     return std::max(LOG_MAXC - 1, logM - LOG_MAXR);
 }
-// Row length of a planned batch's class, whose launches fill the GPU whatever
-// the shape: whole rows up to 2^13 points, then rows of 2^9 (one strided pass
+// Row length of a planned batch's class whose launches fill the GPU (batch_fills)
+// whatever the shape: whole rows up to 2^13 points, then rows of 2^9 (one strided pass
 // before the tensor cores), 2^11 at 2^19.  Measured, us a product in a batch of
 // equal ones: 2^13 points 13: 0.80, 11: 0.88; 2^14 9: 1.29, 5: 1.44, 12 above
 // 1.64; 2^15 9: 2.80, 10: 2.83; 2^16 9: 5.62, 11: 5.65; 2^17 9: 11.31, 12: 11.89;
