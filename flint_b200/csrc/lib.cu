@@ -736,6 +736,22 @@ static bool rows_dependent(size_t points, int logC, int loge = 5)
     return points <= (size_t)1 << 20 && (logC < LOG_MAXC || loge < 5);
 }
 
+// An inverse column pass runs as a dependent of the row pass unless its CTAs
+// would be placed beside row CTAs that leave part of the GPU free, and share SMs:
+// behind row items of 2^13 words (two a SM), fewer than three per SM (dependent
+// against plain: mod 3, a window on 3 2^19 points 67.5 / 61.1 us and a square of
+// 2^20 coefficients 52.6 / 45.3; 2^18 x 2^18 limbs 69.6 / 65.7; with more items 2^19 x
+// 2^19 limbs 108.7 / 110.8, mod a 62-bit n on 3 2^19 points 164.6 / 167.7), and behind
+// configured rows shorter than 2^9 points with columns of 2^6 or more (2^15 points,
+// rows of 2^7: 35.4 / 28.8; with shorter columns, 2^12 points and 2^8, 26.3 / 28.7).
+// Columns of 2^9 points and more have no wait compiled in.
+static bool inv_dependent(const Ctx *X, int logR, int logC, int64_t items, int nv)
+{
+    if (logR >= 9) return false;
+    if (logC < ROWS16_MIN_LOGC) return logR < 6;
+    return nv << logC < 1 << (LOG_MAXC - 1) || items >= 3 * (int64_t)X->nsm;
+}
+
 // the three transform launches shared by every product type; with a batch
 // descriptor array (ninst products of this shape) a, b, ra, rb are ignored;
 // with fz the operands are integer polynomials (an, bn coefficients); with co
@@ -1249,8 +1265,9 @@ static uint32_t *launch_transforms(const Ctx *X, const LaunchShape &L, int np, c
                 dep && rows_dependent((size_t)1 << (S.logR + S.logC), S.logC, loge));
     timing_mark(tr, 2, st);
     if (S.logR > 0)
-        launch_dep(inv, dim3(ci.grid, np, ni), ci.threads, ci.smem, st, dep && S.logR < 9, X->T, ra, S.logC, ci.G, desc,
-                   co ? *co : ChunkOut{nullptr, 0, 0, 0, 0}, fold_inv ? d_scale : nullptr);
+        launch_dep(inv, dim3(ci.grid, np, ni), ci.threads, ci.smem, st,
+                   dep && inv_dependent(X, S.logR, S.logC, (int64_t)(R + Lr.nv - 1) / Lr.nv * np, Lr.nv), X->T, ra, S.logC,
+                   ci.G, desc, co ? *co : ChunkOut{nullptr, 0, 0, 0, 0}, fold_inv ? d_scale : nullptr);
     timing_mark(tr, 3, st);
     return done(ra);
 }
@@ -1278,8 +1295,8 @@ static void launch_transforms3(const Ctx *X, int np, int k, int logMs, const uin
     launch_rows(X, L, 5, ra, rb, logMs - LOGC3, np, nullptr, sq ? 1 : 0, nullptr, 1, rows, st,
                 rows_dependent((size_t)3 << k, LOGC3));
     timing_mark(tr, 2, st);
-    launch_dep(INV_COLS3[r - LOG3_RMIN + (sq ? 6 : 0)], dim3(C / G, np), THREADS3, smem, st, true, X->T, ra, logMs, k,
-               sq ? sc : nullptr);
+    launch_dep(INV_COLS3[r - LOG3_RMIN + (sq ? 6 : 0)], dim3(C / G, np), THREADS3, smem, st,
+               inv_dependent(X, 0, LOGC3, (int64_t)rows * np, 1), X->T, ra, logMs, k, sq ? sc : nullptr);
     timing_mark(tr, 3, st);
 }
 

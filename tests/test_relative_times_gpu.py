@@ -98,3 +98,30 @@ def test_batches_of_few_products(ctx, logM, count):
     fixed = _batch(torch, ctx, n, count, [FB.MulConfig(FB.ROUTE_NTT, 0, 0, logM - 5, 0)] * count)
     torch.cuda.synchronize()
     _ratio_below(torch, lambda s: plain.run(s), lambda s: fixed.run(s), 1.10)
+
+
+def test_configured_short_rows(ctx):
+    """2^15 points in rows of 2^7 against rows of 2^9: 1.18 (with inverse columns
+    placed beside the rows 1.45)."""
+    torch = pytest.importorskip("torch")
+    n = 1 << 14
+    a, b, z = _limbs(torch, n), _limbs(torch, n), _limbs(torch, 2 * n)
+    torch.cuda.synchronize()
+    run = lambda c: lambda s: ctx.mpn_mul_device_config(z.data_ptr(), a.data_ptr(), n, b.data_ptr(), n,
+                                                        FB.MulConfig(FB.ROUTE_NTT, 0, 0, c, 0), s)
+    _ratio_below(torch, run(7), run(9), 1.30, reps=100)
+
+
+def test_squares_modulo_a_small_prime(ctx):
+    """A square mod 3 on one prime against one mod 1000003 on two, 2^20 coefficients
+    on 3 2^19 points: 0.71 (with inverse columns placed beside the rows 0.79)."""
+    torch = pytest.importorskip("torch")
+    n = 1 << 19
+    a = torch.randint(0, 3, (n,), dtype=torch.int64, device="cuda")
+    z = torch.empty(2 * n + 1001, dtype=torch.int64, device="cuda")
+    m = n + 500                                    # a product of 2^20 + 999 coefficients
+    a = torch.cat([a, a[:500]])
+    torch.cuda.synchronize()
+    run = lambda p: lambda s: ctx.nmod_poly_mul_mid_device(z.data_ptr(), 0, 2 * m - 1, a.data_ptr(), m, a.data_ptr(), m,
+                                                           p, s)
+    _ratio_below(torch, run(3), run(1000003), 0.75, reps=100)
