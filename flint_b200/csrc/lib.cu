@@ -748,6 +748,7 @@ static bool rows_dependent(size_t points, int logC, int loge = 5)
 static bool inv_dependent(const Ctx *X, int logR, int logC, int64_t items, int nv)
 {
     if (logR >= 9) return false;
+    if (logR < 5) return true;   // few CTAs of little work: 2^14 points, rows of 2^13, 21.9 / 24.6
     if (logC < ROWS16_MIN_LOGC) return logR < 6;
     return nv << logC < 1 << (LOG_MAXC - 1) || items >= 3 * (int64_t)X->nsm;
 }
@@ -1296,7 +1297,7 @@ static void launch_transforms3(const Ctx *X, int np, int k, int logMs, const uin
                 rows_dependent((size_t)3 << k, LOGC3));
     timing_mark(tr, 2, st);
     launch_dep(INV_COLS3[r - LOG3_RMIN + (sq ? 6 : 0)], dim3(C / G, np), THREADS3, smem, st,
-               inv_dependent(X, 0, LOGC3, (int64_t)rows * np, 1), X->T, ra, logMs, k, sq ? sc : nullptr);
+               inv_dependent(X, r, LOGC3, (int64_t)rows * np, 1), X->T, ra, logMs, k, sq ? sc : nullptr);
     timing_mark(tr, 3, st);
 }
 
