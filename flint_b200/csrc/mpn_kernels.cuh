@@ -229,7 +229,7 @@ __device__ __forceinline__ uint32_t load_residue(const uint64_t* __restrict__ x,
 // it compiled in).
 template <int LOGR, int G>
 __device__ __host__ constexpr bool fwd_cols_dep() { return LOGR < 5 || G < cols_per_tile(LOGR); }
-template <int LOGR, int G, bool FZ, int LC>
+template <int LOGR, int G, bool FZ, int LC, bool DEP>
 __device__ __forceinline__ void
 fwd_cols_body(DevTables T, const uint64_t* __restrict__ a, uint64_t an,
               const uint64_t* __restrict__ b, uint64_t bn,
@@ -418,7 +418,7 @@ fwd_cols_body(DevTables T, const uint64_t* __restrict__ a, uint64_t an,
             gs_contig<5, COL_FMA_ADDS>(xr, c_w32[j], p);
             const uint32_t col = (uint32_t)(i0 + v);
             twist32<LOGR>(xr, col, s, logM, th, tl, P, fsc);
-            if constexpr (fwd_cols_dep<LOGR, G>()) pdl_trigger();
+            if constexpr (DEP) pdl_trigger();
             // rows 32 s .. 32 s + 31 of column col: a pointer bump per row keeps
             // the address arithmetic on the ALU pipe (the FMA pipe is this
             // kernel's busiest unit)
@@ -459,7 +459,7 @@ fwd_cols_body(DevTables T, const uint64_t* __restrict__ a, uint64_t an,
 // the run-time body behind a branch that never takes it for its shape: with
 // that second body the compiler schedules the constant-stride one better
 // (1.21 ms alone, 1.13 ms with it; three bodies in one kernel: 1.24 ms).
-template <int LOGR, int G, bool FZ, int LC = 0>
+template <int LOGR, int G, bool FZ, int LC = 0, bool DEP = fwd_cols_dep<LOGR, G>()>
 __global__ void __launch_bounds__(512)
 k_fwd_cols(DevTables T, const uint64_t* __restrict__ a, uint64_t an,
            const uint64_t* __restrict__ b, uint64_t bn,
@@ -467,11 +467,11 @@ k_fwd_cols(DevTables T, const uint64_t* __restrict__ a, uint64_t an,
            const InstDesc* __restrict__ desc, int np, FzShape fz, const uint32_t* __restrict__ fscale,
            int fmask)
 {
-    if constexpr (fwd_cols_dep<LOGR, G>()) pdl_wait();
+    if constexpr (DEP) pdl_wait();
     if (LC != 0 && logC == LC)
-        fwd_cols_body<LOGR, G, FZ, LC>(T, a, an, b, bn, ra, rb, logC, gcols, desc, np, fz, fscale, fmask);
+        fwd_cols_body<LOGR, G, FZ, LC, DEP>(T, a, an, b, bn, ra, rb, logC, gcols, desc, np, fz, fscale, fmask);
     else
-        fwd_cols_body<LOGR, G, FZ, 0>(T, a, an, b, bn, ra, rb, logC, gcols, desc, np, fz, fscale, fmask);
+        fwd_cols_body<LOGR, G, FZ, 0, DEP>(T, a, an, b, bn, ra, rb, logC, gcols, desc, np, fz, fscale, fmask);
 }
 
 // ---------------------------------------------------------------------------

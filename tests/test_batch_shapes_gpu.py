@@ -44,3 +44,10 @@ def test_mixed_with_configured_and_promoted(ctx):
     _check(ctx, sizes, configs)
     _check(ctx, sizes, configs, promote_small=4)
     _check(ctx, sizes, promote_small=6, max_streams=1, use_graph=False)
+
+
+@pytest.mark.parametrize("logM", [14, 15, 16, 17])
+def test_narrow_column_tiles(ctx, logM):
+    """Columns of 2^5 to 2^8 points in classes small enough for narrow tiles."""
+    n = 1 << (logM - 1)
+    _check(ctx, [(n, n), (n - 5, n - 1000)], [FB.MulConfig(FB.ROUTE_NTT, 0, 0, 9, 0)] * 2)
