@@ -674,10 +674,9 @@ static int batch_logC(int logM)
     if (logM <= 18) return 9;
     return logM == 19 ? 11 : single_logC(logM);
 }
-// Shortest row for a transform of 2^logM points: columns at most 2^11 long,
-// and with 32 or more columns (the column kernel's tiles are up to
-// 2^(14 - logR) columns wide) rows at least one tile wide, which below 2^14
-// points means at most 16 columns.
+// Shortest row for a transform of 2^logM points: columns at most 2^11 long, and
+// below 2^14 points at most 16 of them: longer columns are taken in tiles of up to
+// 2^(13 - logR) columns (cols_per_tile), which the rows must fill.
 static int min_logC(int logM)
 {
     int lo = std::max(MIN_LOGM, logM - LOG_MAXR);
@@ -942,9 +941,10 @@ static int ceil_log2_u64(uint64_t x)
     return l;
 }
 
-// Plan under an explicit configuration (zero fields take the defaults of
-// plan_mpn); every choice is checked against the exactness bound and the
-// kernels' shape limits.
+// Plan under an explicit configuration: zero np and logM take plan_mpn's, a zero
+// logC the row length that the configuration's documentation names (default_logC,
+// not the single_logC of a product without a configuration); every choice is
+// checked against the exactness bound and the kernels' shape limits.
 static int plan_mpn(uint64_t an, uint64_t bn, MulPlan *P);
 static int three_length(uint64_t L, int np, int logM);
 static int split_plan(uint64_t an, uint64_t bn, int logM);

@@ -99,9 +99,10 @@ struct MulShape {
     int G;                 // columns per column-pass tile
 };
 
-// columns per tile for a column length 2^logR: 32 KB tiles (256 threads, four
-// CTAs per SM whose loads, levels and stores overlap), at least 8 columns
-// (32-byte row segments).  Against 64 KB tiles of 512 threads, two per SM, which
+// columns per tile for a column length 2^logR: 32 KB tiles (256 threads; at 57 to 64
+// registers four CTAs per SM, whose loads, levels and stores overlap -- the inverse
+// pass of 2^5-point columns, whole in registers, takes 128 and two), at least 8
+// columns (32-byte row segments).  Against 64 KB tiles of 512 threads, two per SM, which
 // 2^11-point columns keep: columns of 2^8 points (2^20 x 2^20 limbs) forward 74.2 ->
 // 68.3 us, inverse 36.6 -> 32.0; 2^9 137.7 -> 125.7, 61.6 -> 57.3; 2^10 284.0 ->
 // 282.2, 135.0 -> 128.8.
@@ -213,6 +214,14 @@ __device__ __forceinline__ uint32_t load_residue(const uint64_t* __restrict__ x,
     }
 }
 
+// Forward column instances that may run as programmatic dependents: short
+// columns and narrow tiles, which only launches of a few CTAs per SM take.  The wide
+// ones serve large products, where a launch gap is nothing and the wait's memory
+// barrier costs the schedule of the loads (2^25-point forward pass 1.13 -> 1.5 ms
+// with it compiled in).
+template <int LOGR, int G>
+__device__ __host__ constexpr bool fwd_cols_dep() { return LOGR < 5 || G < cols_per_tile(LOGR); }
+
 // ---------------------------------------------------------------------------
 // Column pass, forward: split + length-R transforms + twist.
 // grid = (np, C / G, operands) -- the prime index varies fastest so that the
@@ -222,13 +231,7 @@ __device__ __forceinline__ uint32_t load_residue(const uint64_t* __restrict__ x,
 // smem = padw(R * G) words.
 // LC != 0: the row length 2^LC is a compile-time constant (logC == LC), so
 // the strided stores take immediate offsets instead of address arithmetic.
-// Instances that may run as programmatic dependents: short columns and narrow
-// tiles, which only launches of a few CTAs per SM take.  The wide ones serve
-// large products, where a launch gap is nothing and the wait's memory barrier
-// costs the schedule of the loads (2^25-point forward pass 1.13 -> 1.5 ms with
-// it compiled in).
-template <int LOGR, int G>
-__device__ __host__ constexpr bool fwd_cols_dep() { return LOGR < 5 || G < cols_per_tile(LOGR); }
+// DEP: the kernel may run as a programmatic dependent.
 template <int LOGR, int G, bool FZ, int LC, bool DEP>
 __device__ __forceinline__ void
 fwd_cols_body(DevTables T, const uint64_t* __restrict__ a, uint64_t an,

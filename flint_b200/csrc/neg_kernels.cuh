@@ -9,12 +9,13 @@
 // t -> omega t, omega^m = -1 (omega of order 2m):
 //
 //   k_neg_split     digit i -> residue, times omega^i        [per prime]
-//   k_rows          length-m forward transforms of x and y, pointwise product
+//   k_rows          length-m forward transforms of x and y, pointwise product,
 //                   inverse transform (the mpn row kernel, one row per product)
 //   k_neg_finish    per product: untwist omega^-i with the CRT cofactor
-//                   inverse and the normalisation 2^128 / m, add a bias B = 2^(2b + log m) so every coefficient
-//                   is non-negative, CRT, recompose sum V_i 2^(b i) with the
-//                   carries, add (-biaspoly mod 2^N + 1), fold mod 2^N + 1.
+//                   inverse and the normalisation 2^128 / m, add a bias
+//                   B = 2^(2b + log m) so every coefficient is non-negative, CRT,
+//                   recompose sum V_i 2^(b i) with the carries, add
+//                   (-biaspoly mod 2^N + 1), fold mod 2^N + 1.
 //
 // The staged variant (a cached transform of y) runs k_rows_fwd on x,
 // k_neg_pointwise against the cached spectrum and k_rows_inv instead of k_rows.

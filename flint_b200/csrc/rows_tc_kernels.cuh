@@ -7,9 +7,9 @@
 // words as 256 rows of 32 residues, two 128-row A tiles, and the sums come back
 // from TMEM to the thread that owns the row.
 //
-// What bounds it: issue slots and latency at 16 warps per SM (issue 55%, FMA-heavy
-// pipe 51%, ALU 48%, tensor pipe 8% of cycles; 161 instructions a point against
-// 168): the five levels cost 9 instructions a word for tc_reduce instead of 15 of
+// What bounds it: issue slots and latency at 16 warps per SM (2^13-point rows of a
+// 2^23-point product: issue 53% of cycles, FMA-heavy pipe 53%, ALU 48%, tensor pipe
+// 8%; 159 instructions a point against 168; profiles/rows_tc_mpn22.md): the five levels cost 9 instructions a word for tc_reduce instead of 15 of
 // butterflies.  512 threads of 16 words at 64 registers were slower (834 against
 // 705 us on a 2^24-point product: the second vector of a strided pass no longer
 // fits, so its twiddles are loaded twice).
@@ -265,7 +265,10 @@ k_rows_tc(DevTables T, uint32_t* __restrict__ ra, const uint32_t* __restrict__ r
 
         uint32_t breg[32];
         if (squaring == 0) {
-            if constexpr (REM == 5) {   // one pass of five levels: two vectors would spill
+            // One pass of five levels: a vector at a time, and the instance still spills
+            // (2^10-point rows: 236 bytes a thread; the other lengths none).  Two
+            // vectors together would need twice the registers.
+            if constexpr (REM == 5) {
                 tc_gs_passes<LOGC, 1, 5, (1 << (LOGC - 1)), REM>(sb, sb, nv, twf, p);
                 tc_gs_passes<LOGC, 1, 5, (1 << (LOGC - 1)), REM>(sa, sa, nv, twf, p);
             } else {

@@ -56,7 +56,9 @@ def _req(r):
 
 def default_config(r):
     """The fixed rule (the method without the model): transform route, fewest
-    primes, shortest transform, longest rows."""
+    primes, shortest transform, and the row length that a configuration's open
+    field documents.  A product without a configuration takes rows fitted to the
+    kernels and 3 2^k lengths instead, which are faster."""
     kind, an, bn, aw, bw = _req(r)
     return resolve_config(kind, an, bn, None, aw, bw)
 
