@@ -226,6 +226,10 @@ struct Ctx {
     uint32_t *d_scale = nullptr;          // [np][logM][MAX_NP] pointwise scales
     int *d_err = nullptr;
     int *h_err = nullptr;                 // pinned copy of *d_err, read after a host-pointer product
+    // whether a kernel that can set *d_err has been launched: on the context's
+    // stream since the flag was last read, or ever on another one (whose kernels
+    // may end after a read)
+    mutable bool err_own = false, err_foreign = false;
     unsigned long long *d_ticket = nullptr;
     unsigned long long ticket_base = 0;
     uint32_t *d_status = nullptr;
@@ -714,6 +718,12 @@ static LaunchShape make_shape(int logM, int logC = -1)
     return L;
 }
 
+// A kernel that can set the error flag is about to be launched on st.
+static void note_err_launch(const Ctx *X, cudaStream_t st)
+{
+    (st == X->stream ? X->err_own : X->err_foreign) = true;
+}
+
 // Launch as a programmatic dependent of the kernel before it on the stream
 // (dep), or plainly.
 template <typename... P, typename... A>
@@ -1137,6 +1147,7 @@ static void launch_rows(const Ctx *X, const LaunchShape &L, int loge, uint32_t *
     // 2^14-point rows would need twice its TMEM and shared memory, and launches
     // short of warps run 16 points per thread.
     if (loge == 5 && logC >= ROWS_TC_MIN_LOGC && (L.nv << logC) == TC_WORDS && X->T.tcw) {
+        note_err_launch(X, st);
         launch_dep(ROWS_TC[logC], (unsigned)std::min<int64_t>(items, 2 * X->nsm), TC_THREADS, TC_ROWS_SMEM, st, dep, X->T,
                    ra, rb, logR, L.nv, np, scale, squaring, desc, ninst, rows);
         return;
@@ -1349,6 +1360,7 @@ static int mpn_mul_basecase_enqueue(Ctx *X, uint64_t *z, const uint64_t *a, uint
     timing_mark(tr, 1, st);
     timing_mark(tr, 2, st);
     timing_mark(tr, 3, st);
+    note_err_launch(X, st);
     k_crt_carry<0, THREADS><<<tiles, THREADS, 0, st>>>((const uint32_t *)sums, logM, L, zn, z, X->crt[5],
                                                        X->d_status, X->d_ticket, X->ticket_base, X->epoch,
                                                        X->d_err, nullptr, nullptr, 0ull);
@@ -1566,6 +1578,7 @@ static int mpn_mul_enqueue(Ctx *X, uint64_t *z, const uint64_t *a, uint64_t an,
     // tiles take their index from the ticket counter, so consecutive launches
     // with the same ticket base continue one carry chain: tile k's look-back
     // finds tile k - 1 finished by an earlier launch
+    note_err_launch(X, st);
     const int nch = (chunks && !window) ? std::max(1, std::min<int>(chunks->chunks, (int)tiles)) : 1;
     for (int c = 0; c < nch; c++) {
         const size_t t0 = tiles * c / nch, t1 = tiles * (c + 1) / nch;
@@ -1603,7 +1616,24 @@ static int take_device_error(Ctx *X)
 // (through the pinned word: one copy, no staging).
 static int check_device_error(Ctx *X)
 {
+    X->err_own = false;
     CU(cudaMemcpyAsync(X->h_err, X->d_err, sizeof(int), cudaMemcpyDeviceToHost, X->stream));
+    CU(cudaStreamSynchronize(X->stream));
+    return take_device_error(X);
+}
+
+// The end of a host-pointer call whose kernels are queued on the context's
+// stream: the error flag if one of them can have set it, the result home, the wait.
+// The flag goes first, since a copy to pageable memory returns when it is done, and
+// a second round trip behind it would cost a short call 7 us of 38.
+static int finish_host_call(Ctx *X, void *z, const void *dz, size_t bytes)
+{
+    if (X->err_own || X->err_foreign)
+        CU(cudaMemcpyAsync(X->h_err, X->d_err, sizeof(int), cudaMemcpyDeviceToHost, X->stream));
+    else
+        *X->h_err = 0;
+    X->err_own = false;
+    CU(cudaMemcpyAsync(z, dz, bytes, cudaMemcpyDeviceToHost, X->stream));
     CU(cudaStreamSynchronize(X->stream));
     return take_device_error(X);
 }
@@ -1735,6 +1765,7 @@ static int mpn_mul_host_finish(Ctx *X, gpu_ulong *z, gpu_ulong an, gpu_ulong bn,
     else if (X->copy_stream) CU(cudaStreamSynchronize(X->copy_stream));
     if (an + bn > lo && std::min<gpu_ulong>(hi, an + bn) > lo) {
         // the flag was copied behind the last download
+        X->err_own = false;
         rc = take_device_error(X);
         if (rc) return rc;
     } else {
@@ -2321,6 +2352,7 @@ int gpu_test_crt_lookback_timeout(gpu_mpn_ctx_t R)
         CU(cudaMemsetAsync(X->d_status, 0, X->status_cap * sizeof(uint32_t), st));
         X->epoch = 1;
     }
+    note_err_launch(X, st);
     k_crt_carry<5, CRT_THREADS><<<1, CRT_THREADS, 0, st>>>(X->d_res, logM, M - 1, M, dz, X->crt[5], X->d_status,
                                                           X->d_ticket, X->ticket_base - 1, X->epoch, X->d_err,
                                                           nullptr, nullptr, 0ull);
@@ -2342,6 +2374,8 @@ int gpu_test_set_device_error_bits(gpu_mpn_ctx_t R, int bits)
     if (!X) return set_error(GPU_FFT_SMALL_EINVAL, "context not initialised");
     int rc = bind_device(X);
     if (rc) return rc;
+    if (!(bits & 256)) note_err_launch(X, X->stream);
+    bits &= 255;
     CU(cudaMemcpyAsync(X->d_err, &bits, sizeof(int), cudaMemcpyHostToDevice, X->stream));
     CU(cudaStreamSynchronize(X->stream));
     return 0;

@@ -493,7 +493,8 @@ GPU_FFT_SMALL_API int gpu_fmpz_poly_mul_mid_device_list(gpu_mpn_ctx_t R, const g
    and clears it.  gpu_test_set_device_error_bits sets the bits a kernel would:
    1 a carry look-back (as the former), 2 a row pass's wait for a matrix product
    (both GPU_FFT_SMALL_ETIMEOUT, each with its own message), 4 a row pass whose
-   shared memory is misaligned (GPU_FFT_SMALL_ECUDA).  gpu_test_pipe_slot_ctx returns the context behind slot
+   shared memory is misaligned (GPU_FFT_SMALL_ECUDA); plus 256: as a kernel of an
+   earlier device-pointer call that ends only now.  gpu_test_pipe_slot_ctx returns the context behind slot
    `slot` of a pipeline (the impl of a gpu_mpn_ctx_t), or NULL. */
 GPU_FFT_SMALL_API int gpu_test_crt_lookback_timeout(gpu_mpn_ctx_t R);
 GPU_FFT_SMALL_API int gpu_test_set_device_error(gpu_mpn_ctx_t R);

@@ -78,3 +78,27 @@ def test_message_names_the_kernel(ctx, bits, code, words):
     assert all(w in str(e.value) for w in words)
     assert ("carry" in str(e.value)) == bool(bits & 1)
     ctx.check()
+
+
+def test_error_of_an_earlier_device_call_is_not_lost():
+    """A host call that launches no kernel which can set the flag skips reading it,
+    but not after a device-pointer call on another stream, whose kernels may end
+    after any number of reads."""
+    torch = pytest.importorskip("torch")
+    with FB.MpnCtx() as c:
+        s = torch.cuda.Stream()
+        a = torch.randint(-(1 << 62), 1 << 62, (100,), dtype=torch.int64, device="cuda")
+        z = torch.empty(200, dtype=torch.int64, device="cuda")
+        torch.cuda.synchronize()
+        c.mpn_mul_device(z.data_ptr(), a.data_ptr(), 100, a.data_ptr(), 100, s.cuda_stream)
+        x = O.rand_below(1, 50, MOD)
+        want = O.port_nmod_mul_mid(0, 99, x, x, MOD)
+        for _ in range(2):
+            assert (c.nmod_poly_mul_mid(0, 99, x, x, MOD) == want).all()
+        s.synchronize()
+        FB._check(FB.lib().gpu_test_set_device_error_bits(c.ptr, 1 + 256))
+        c2 = FB.lib().gpu_mpn_ctx_check
+        with pytest.raises(FB.GpuFftSmallError):
+            c.nmod_poly_mul_mid(0, 99, x, x, MOD)
+        assert (c.nmod_poly_mul_mid(0, 99, x, x, MOD) == want).all()
+        assert c2(c.ptr, None) == FB.OK
