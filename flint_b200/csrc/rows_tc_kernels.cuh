@@ -9,10 +9,10 @@
 //
 // What bounds it: issue slots and latency at 16 warps per SM (2^13-point rows of a
 // 2^23-point product: issue 53% of cycles, FMA-heavy pipe 53%, ALU 48%, tensor pipe
-// 8%; 159 instructions a point against 168): the five levels cost 9 instructions a word for tc_reduce instead of 15 of
-// butterflies.  512 threads of 16 words at 64 registers were slower (834 against
-// 705 us on a 2^24-point product: the second vector of a strided pass no longer
-// fits, so its twiddles are loaded twice).
+// 8%; 159 instructions a point against 168): the five levels cost 9 instructions a
+// word for tc_reduce instead of 15 of butterflies.  512 threads of 16 words at 64
+// registers were slower (834 against 705 us on a 2^24-point product: the second
+// vector of a strided pass no longer fits, so its twiddles are loaded twice).
 //
 // Row buffers hold position pos at word tc_swz(pos), which is the operand
 // layout and needs no padding: every strided access of a warp is 32 consecutive
